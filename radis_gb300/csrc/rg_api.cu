@@ -655,7 +655,8 @@ int ensure_workspace(Work& W, int n_nodes, cudaStream_t st) {
 }
 
 // Entries of the scatter's per-tile line-range table: at least the tiles of
-// any CTA, whatever tile width the shape takes (>= 32 columns), so at most
+// any CTA, whatever tile width the shape may take (the rounds of tiles of the
+// largest width, >= 32 columns), so at most
 // ceil(ceil(n_v / 32) / sms) while the grid is one CTA per SM, and never more
 // than kScatMaxTilesPerCta (more CTAs are launched past that); even.
 int scatter_rng_cap(int64_t n_v, int sms) {
@@ -664,12 +665,19 @@ int scatter_rng_cap(int64_t n_v, int sms) {
     return (cap + 1) & ~1;
 }
 
+// Lines per column from which the scatter keeps copies of a small tile.
+constexpr double kScatCopyDensity = 4.0;
+
 // Shape of the persistent scatter (one 1024-thread CTA per SM): TMA ring
-// stages, chunk (lines) and tile width (columns, a multiple of 32 for the bank
-// swizzle), the widest tile that fits beside the ring, the line-range table
-// (rng_cap entries) and coef_bytes of skeleton projection data (0 without).
-int scatter_shape(int n_nodes, bool wide, size_t coef_bytes, int rng_cap, int* chunk, int* TK, int* stages,
-                  size_t* smem) {
+// stages, chunk (lines), tile width (columns), row pitch, copies of the tile
+// and dynamic shared memory, beside the line-range table (rng_cap entries) and
+// coef_bytes of skeleton projection data (0 without).
+struct ScatterShape {
+    int chunk = 0, TK = 0, pitch = 0, stages = 0, copies = 1, copy_words = 0;
+    size_t smem = 0;
+};
+int scatter_shape(int n_nodes, bool wide, size_t coef_bytes, int rng_cap, int64_t n_v, int sms, double lines_per_col,
+                  ScatterShape* sh) {
     size_t avail = 0;
     RG(scatter_smem_optin(&avail, wide));
     const size_t word = wide ? 8 : 4;   // bytes per tile cell
@@ -678,12 +686,27 @@ int scatter_shape(int n_nodes, bool wide, size_t coef_bytes, int rng_cap, int* c
         if (fixed >= avail) return 0;
         return std::min(1024, ((int)((avail - fixed) / (word * (size_t)n_nodes)) - 1) / 32 * 32);
     };
-    auto take = [&](int S, int ch, int tk) {
-        *chunk = ch;
-        *TK = tk;
-        *stages = S;
-        *smem = scatter_fixed_smem(ch, S, rng_cap) + scatter_coef_offset((size_t)n_nodes * (tk + 1), word) +
-                coef_bytes;
+    auto take = [&](int S, int ch, int tk_max) {
+        sh->chunk = ch;
+        sh->stages = S;
+        // the tiles of the fewest rounds of one tile per CTA, all equally wide:
+        // a window of few columns still reaches every SM (5001 columns, 2400
+        // lines each, 64-bit sums: 5 tiles of 1024 columns took 8.9 ms, 152 of 33
+        // take 0.18 ms), and the last round is full
+        const int64_t rounds = (n_v + (int64_t)sms * tk_max - 1) / ((int64_t)sms * tk_max);
+        const int64_t per = (n_v + rounds * sms - 1) / (rounds * sms);
+        sh->TK = (int)std::min<int64_t>(tk_max, per <= 64 ? per : (per + 15) / 16 * 16);
+        sh->pitch = (sh->TK + 31) / 32 * 32 + 1;
+        auto bytes = [&](int copies) {
+            return scatter_fixed_smem(ch, S, rng_cap) + coef_bytes +
+                   scatter_coef_offset((size_t)copies * scatter_copy_words(n_nodes, sh->pitch, wide, copies));
+        };
+        // copies of a small tile for lists of many lines per column: the lanes
+        // of a warp (sorted lines) then meet in one cell less often
+        sh->copies = 1;
+        while (lines_per_col >= kScatCopyDensity && sh->copies < 8 && bytes(2 * sh->copies) <= avail) sh->copies *= 2;
+        sh->copy_words = scatter_copy_words(n_nodes, sh->pitch, wide, sh->copies);
+        sh->smem = bytes(sh->copies);
         return RG_OK;
     };
     // GB300 sweeps (CO2 5M / 128 nodes, H2O 100M / 288 nodes): one line per
@@ -699,6 +722,18 @@ int scatter_shape(int n_nodes, bool wide, size_t coef_bytes, int rng_cap, int* c
     return fail(RG_ERR_RANGE, "LDM grid of %d nodes does not fit a shared-memory tile", n_nodes);
 }
 
+// Mean lines per grid column of a list over its own range (all the host knows
+// of the density without reading the index back).
+double mean_lines_per_col(const rg_lines* L, double dv) {
+    double lo = std::numeric_limits<double>::infinity(), hi = -lo;
+    for (int i = 0; i < L->n_iso; ++i) {
+        lo = std::min(lo, L->env.lv_min[i]);
+        hi = std::max(hi, L->env.lv_max[i]);
+    }
+    const double span = std::exp(hi) - std::exp(lo);
+    return (double)L->n * dv / std::max(span, dv);
+}
+
 // Shared-memory bytes of the skeleton projection beside the scatter's tile:
 // the tensor-core flush's section (32-bit tiles, where the grid has one) or
 // the FP32 coefficients.
@@ -708,9 +743,10 @@ size_t fuse_smem_bytes(const ProjArgs* fuse, bool wide) {
     return sizeof(float) * (size_t)fuse->n_nodes * fuse->rows_pad;
 }
 
-// fuse: the skeleton projection done by the scatter's flush (nullable).
+// fuse: the skeleton projection done by the scatter's flush (nullable); smem
+// (nullable): the launch's dynamic shared memory.
 int build_scatter_args(const rg_lines* L, const Work& W, const rg_conditions* c, const SpecHost& s, bool wide,
-                       const ProjArgs* fuse, ScatterArgs* a) {
+                       const ProjArgs* fuse, ScatterArgs* a, size_t* smem) {
     const rg_grid& g = s.grid;
     std::memset(a, 0, sizeof *a);
     a->v0 = L->v0;
@@ -742,9 +778,17 @@ int build_scatter_args(const rg_lines* L, const Work& W, const rg_conditions* c,
             a->proj_nr = fuse->flush_nr;
         }
     }
-    size_t smem_unused;
     a->rng_cap = scatter_rng_cap(W.desc.n_v, L->ctx->sms);
-    RG(scatter_shape(s.n_nodes, wide, coef_bytes, a->rng_cap, &a->chunk, &a->TK, &a->stages, &smem_unused));
+    ScatterShape sh;
+    RG(scatter_shape(s.n_nodes, wide, coef_bytes, a->rng_cap, W.desc.n_v, L->ctx->sms,
+                     mean_lines_per_col(L, W.desc.dv), &sh));
+    a->chunk = sh.chunk;
+    a->TK = sh.TK;
+    a->pitch = sh.pitch;
+    a->stages = sh.stages;
+    a->copies = sh.copies;
+    a->copy_words = sh.copy_words;
+    if (smem) *smem = sh.smem;
     a->n_tiles = (int)((W.desc.n_v + a->TK - 1) / a->TK);
     a->cmax = W.cmax_dev;
     a->err = W.err;
@@ -1250,10 +1294,7 @@ int take_err(Work& W) {
 // and dynamic shared memory.
 int scatter_launch_shape(const rg_lines* L, const Work& W, const rg_conditions* c, const SpecHost& s, bool wide,
                          const ProjArgs* fuse, ScatterArgs* sa, int* grid, size_t* smem) {
-    RG(build_scatter_args(L, W, c, s, wide, fuse, sa));
-    int ch_unused, tk_unused, st_unused;
-    RG(scatter_shape(s.n_nodes, wide, fuse_smem_bytes(fuse, wide), sa->rng_cap, &ch_unused, &tk_unused, &st_unused,
-                     smem));
+    RG(build_scatter_args(L, W, c, s, wide, fuse, sa, smem));
     const int sms = L->ctx->sms;
     *grid = std::max(std::min(sa->n_tiles, sms), (sa->n_tiles + kScatMaxTilesPerCta - 1) / kScatMaxTilesPerCta);
     if ((sa->n_tiles + *grid - 1) / *grid > sa->rng_cap)
@@ -1471,7 +1512,7 @@ int enqueue_spectrum(const rg_lines* L, Work& W, const rg_conditions* c, const S
 int fill_grad_args(const rg_lines* L, const Work& W, const rg_conditions* c, const SpecHost& s,
                    const double* dlnq_dT, GradArgs* g) {
     std::memset(g, 0, sizeof *g);
-    RG(build_scatter_args(L, W, c, s, false, nullptr, &g->s));
+    RG(build_scatter_args(L, W, c, s, false, nullptr, &g->s, nullptr));
     if (!(c->x > 0)) return fail(RG_ERR_ARG, "derivatives need a mole fraction x > 0");
     const double T = c->T, p = c->p_bar;
     g->n_lines = L->n;

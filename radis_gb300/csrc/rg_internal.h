@@ -119,7 +119,10 @@ struct ScatterArgs {
     int col_off;
     int col_count;
     int n_v;
-    int TK;               // columns per tile (multiple of 8)
+    int TK;               // columns per tile
+    int pitch;            // words per tile row: 1 (mod 32), >= TK + 1
+    int copies;           // copies of the tile (1, 2, 4 or 8): lane l adds into copy l mod copies
+    int copy_words;       // words from one copy to the next
     int n_nodes;          // padded to even
     int NG, NL;
     int64_t row_stride;
@@ -186,9 +189,17 @@ RG_HD inline size_t flush_tc_bytes(int ks, int nr) { return (size_t)ks * nr * 51
 RG_HD inline size_t scatter_fixed_smem(int chunk, int stages, int rng_cap) {
     return stages * scatter_stage_bytes(chunk) + 16 * kScatMaxStages + 8 * (size_t)rng_cap;
 }
-// byte offset of the flush coefficients (skeleton layout) after a tile of
-// `words` accumulator words of `word` bytes
-RG_HD inline size_t scatter_coef_offset(size_t words, size_t word) { return (words * word + 15) / 16 * 16; }
+// 32-bit words of one copy of a tile of n_nodes rows (64-bit accumulator: the
+// low words' plane, then the high words'); copies beyond the first start 4
+// words (mod 32) further, so that the same cell of the eight copies lies in
+// eight distinct groups of four banks
+RG_HD inline int scatter_copy_words(int n_nodes, int pitch, bool wide, int copies) {
+    const int w = n_nodes * pitch * (wide ? 2 : 1);
+    return copies > 1 ? (w - 4 + 31) / 32 * 32 + 4 : w;
+}
+// byte offset of the flush coefficients (skeleton layout) after `words`
+// 32-bit accumulator words
+RG_HD inline size_t scatter_coef_offset(size_t words) { return (words * 4 + 15) / 16 * 16; }
 
 struct ColFftArgs {       // K2 (forward column FFT) and K4 (inverse column FFT)
     FftLen f1;

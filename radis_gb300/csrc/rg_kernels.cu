@@ -437,7 +437,7 @@ __global__ void k_col_cmax(const int64_t* __restrict__ col_start, int col_off, i
 // ---------------------------------------------------------------------------
 // K1: fused line scaling + LDM scatter into a shared-memory tile
 // ---------------------------------------------------------------------------
-// Tile layout [node][TK + 1]: the odd row pitch puts column c of node n on
+// Tile layout [node][pitch], pitch 1 (mod 32): column c of node n lies in
 // bank (n + c) mod 32.  The lanes of a warp hold neighbouring (sorted) lines,
 // i.e. the same few columns at scattered nodes, so their atomics spread over
 // the banks, and every address is a row base plus a column offset.
@@ -589,25 +589,40 @@ __device__ __forceinline__ float line_intensity(const ScatterArgs& a, float v0, 
     return ex2(arg) * (1.f - ex2(-a.stim_c * v0));
 }
 
-// Fixed-point words of the tile accumulator: 32 bits (one native shared
-// integer atomic per add) or 64 bits for dense columns (see fx_wide).
-template <typename Acc> struct Fx;
-template <> struct Fx<unsigned> {
+// Fixed-point accumulators of the tile: 32-bit words, or 64-bit sums for dense
+// columns (see fx_wide) held as two planes of 32-bit words `hi_off` words
+// apart.  Shared memory has native 32-bit integer adds only (a 64-bit
+// atomicAdd runs as a compare-and-swap loop: 6.6 rounds per add on a band core
+// of 2400 lines per column), so a 64-bit add is a native add of the low word
+// and one of the high word plus the carry that the old low word tells, left
+// out when it is zero.  Integer sums: exact and order-independent.
+template <bool W> struct Fx;
+template <> struct Fx<false> {
     static constexpr int kWidth = 31;
-    __device__ static unsigned to_fx(float v) { return __float2uint_rn(v); }
-    __device__ static float to_float(unsigned w) { return __uint2float_rn(w); }
+    __device__ static void add(unsigned* t, int, float v) { atomicAdd(t, __float2uint_rn(v)); }
+    __device__ static float value(const unsigned* t, int) { return __uint2float_rn(*t); }
 };
-template <> struct Fx<unsigned long long> {
+template <> struct Fx<true> {
     static constexpr int kWidth = 63;
-    __device__ static unsigned long long to_fx(float v) { return __float2ull_rn(v); }
-    __device__ static float to_float(unsigned long long w) { return __ull2float_rn(w); }
+    __device__ static void add(unsigned* t, int hi_off, float v) {
+        const unsigned long long u = __float2ull_rn(v);
+        const unsigned lo = (unsigned)u;
+        const unsigned old = atomicAdd(t, lo);
+        const unsigned hi = (unsigned)(u >> 32) + (old + lo < old ? 1u : 0u);
+        if (hi) atomicAdd(t + hi_off, hi);
+    }
+    __device__ static float value(const unsigned* t, int hi_off) {
+        return __ull2float_rn(((unsigned long long)t[hi_off] << 32) | *t);
+    }
 };
 
-// Scale + scatter of the lines of one staged chunk into the tile accumulator.
-template <typename Acc>
+// Scale + scatter of the lines of one staged chunk into the tile accumulator
+// (`tile`: this lane's copy).
+template <bool W>
 __device__ __forceinline__ unsigned scatter_chunk(const ScatterArgs& a, const Stage& st, int count, int k_start,
-                                                  int tk, Acc* tile, float fxs, int t0, int nt) {
+                                                  int tk, unsigned* tile, float fxs, int t0, int nt) {
     unsigned counted = 0;
+    const int hi_off = a.n_nodes * a.pitch;
     for (int j = t0; j < count; j += nt) {
         const float2 v = st.v0[j];
         const float dl = st.dl ? st.dl[j] : 0.f;
@@ -631,20 +646,20 @@ __device__ __forceinline__ unsigned scatter_chunk(const ScatterArgs& a, const St
         const float w10 = tG - w11;          // tG (1 - tL)
         const float w01 = tL - w11;          // (1 - tG) tL
         const float w00 = 1.f - tG - w01;    // (1 - tG)(1 - tL)
-        const int pitch = a.TK + 1;
+        const int pitch = a.pitch;
         const int dL = a.NL * pitch;                          // next wG node
-        Acc* t = tile + (l0 * a.NL + m0) * pitch + c0;   // (l0, m0) at column c0
+        unsigned* t = tile + (l0 * a.NL + m0) * pitch + c0;   // (l0, m0) at column c0
         if (own0) {
-            atomicAdd(t, Fx<Acc>::to_fx(I0 * w00));
-            atomicAdd(t + pitch, Fx<Acc>::to_fx(I0 * w01));
-            atomicAdd(t + dL, Fx<Acc>::to_fx(I0 * w10));
-            atomicAdd(t + dL + pitch, Fx<Acc>::to_fx(I0 * w11));
+            Fx<W>::add(t, hi_off, I0 * w00);
+            Fx<W>::add(t + pitch, hi_off, I0 * w01);
+            Fx<W>::add(t + dL, hi_off, I0 * w10);
+            Fx<W>::add(t + dL + pitch, hi_off, I0 * w11);
         }
         if (own1) {
-            atomicAdd(t + 1, Fx<Acc>::to_fx(I1 * w00));
-            atomicAdd(t + 1 + pitch, Fx<Acc>::to_fx(I1 * w01));
-            atomicAdd(t + 1 + dL, Fx<Acc>::to_fx(I1 * w10));
-            atomicAdd(t + 1 + dL + pitch, Fx<Acc>::to_fx(I1 * w11));
+            Fx<W>::add(t + 1, hi_off, I1 * w00);
+            Fx<W>::add(t + 1 + pitch, hi_off, I1 * w01);
+            Fx<W>::add(t + 1 + dL, hi_off, I1 * w10);
+            Fx<W>::add(t + 1 + dL + pitch, hi_off, I1 * w11);
         }
     }
     return counted;
@@ -652,12 +667,32 @@ __device__ __forceinline__ unsigned scatter_chunk(const ScatterArgs& a, const St
 
 // Zero `words` accumulator words from thread `i0` in steps of `step` threads,
 // 16 bytes per store (the tile starts on a 16-byte boundary).
-template <typename Acc>
-__device__ __forceinline__ void zero_tile(Acc* tile, int words, int i0, int step) {
-    const int n16 = (int)(((size_t)words * sizeof(Acc)) >> 4);
+__device__ __forceinline__ void zero_tile(unsigned* tile, int words, int i0, int step) {
+    const int n16 = words >> 2;
     uint4* z = reinterpret_cast<uint4*>(tile);
     for (int i = i0; i < n16; i += step) z[i] = make_uint4(0u, 0u, 0u, 0u);
-    for (int i = (int)(((size_t)n16 << 4) / sizeof(Acc)) + i0; i < words; i += step) tile[i] = 0;
+    for (int i = (n16 << 2) + i0; i < words; i += step) tile[i] = 0;
+}
+
+// Sum the tile's copies into the first one (integer sums: exact).
+template <bool W>
+__device__ __forceinline__ void fold_copies(const ScatterArgs& a, unsigned* tile, int i0, int step) {
+    const int n = a.n_nodes * a.pitch;
+    for (int i = i0; i < n; i += step) {
+        if constexpr (W) {
+            unsigned long long s = 0;
+            for (int c = 0; c < a.copies; ++c) {
+                const unsigned* t = tile + c * a.copy_words + i;
+                s += ((unsigned long long)t[n] << 32) | t[0];
+            }
+            tile[i] = (unsigned)s;
+            tile[n + i] = (unsigned)(s >> 32);
+        } else {
+            unsigned s = 0;
+            for (int c = 0; c < a.copies; ++c) s += tile[c * a.copy_words + i];
+            tile[i] = s;
+        }
+    }
 }
 
 // Skeleton rows of a finished 32-bit tile on the tensor cores: Y^T[columns x
@@ -727,10 +762,9 @@ __device__ __forceinline__ void flush_tc(const ScatterArgs& a, const unsigned* t
 // buffer; warps meet only at tile boundaries (a named barrier of the consumer
 // warps) to flush the finished tile to HBM with plain stores.  Every wait is
 // bounded; a wait that gives up sets the error flag and the CTA stops after
-// the copies it issued have landed (bounded).  Acc: the 32- or 64-bit
-// fixed-point word of the tile.  U: unrolling of the tensor-core flush's node
+// the copies it issued have landed (bounded).  W: 64-bit sums.  U: unrolling of the tensor-core flush's node
 // steps (4 where registers allow, 1 in the kernel that holds both variants).
-template <typename Acc, int U = 4>
+template <bool W, int U = 4>
 __device__ __forceinline__ void scatter_body(const ScatterArgs& a) {
     extern __shared__ __align__(128) unsigned char smem[];
     const int ch = a.chunk;
@@ -739,11 +773,12 @@ __device__ __forceinline__ void scatter_body(const ScatterArgs& a) {
     uint64_t* full = reinterpret_cast<uint64_t*>(smem + S * sb);
     uint64_t* empty = full + kScatMaxStages;
     int2* rng = reinterpret_cast<int2*>(smem + S * sb + 16 * kScatMaxStages);
-    Acc* tile = reinterpret_cast<Acc*>(smem + scatter_fixed_smem(ch, S, a.rng_cap));
-    const int pitch = a.TK + 1;
+    unsigned* tile = reinterpret_cast<unsigned*>(smem + scatter_fixed_smem(ch, S, a.rng_cap));
+    const int pitch = a.pitch;
+    const int hi_off = a.n_nodes * pitch;
     const int G = gridDim.x;
     const int nq = (a.n_tiles - (int)blockIdx.x + G - 1) / G;   // tiles of this CTA (<= a.rng_cap)
-    const int n_words = a.n_nodes * pitch;
+    const int n_words = a.copies * a.copy_words;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int n_cons_warps = (blockDim.x >> 5) - 1;
 
@@ -764,9 +799,9 @@ __device__ __forceinline__ void scatter_body(const ScatterArgs& a) {
     // [node][row] or (32-bit tiles) the tensor-core flush's B fragments and
     // node table
     float* coef = reinterpret_cast<float*>(reinterpret_cast<unsigned char*>(tile) +
-                                           scatter_coef_offset(n_words, sizeof(Acc)));
+                                           scatter_coef_offset(n_words));
     const bool proj = a.proj_coef != nullptr;
-    const bool proj_tc = sizeof(Acc) == 4 && proj && a.proj_frag != nullptr;
+    const bool proj_tc = !W && proj && a.proj_frag != nullptr;
     const int n_frag = proj_tc ? a.proj_ks * a.proj_nr * 32 : 0;
     const float4* frag_s = reinterpret_cast<const float4*>(coef);
     const int2* offs_s = reinterpret_cast<const int2*>(frag_s + n_frag);
@@ -816,11 +851,12 @@ __device__ __forceinline__ void scatter_body(const ScatterArgs& a) {
     }
 
     // consumers
-    const float fxs = fx_scale_of(*a.cmax, Fx<Acc>::kWidth);
+    const float fxs = fx_scale_of(*a.cmax, Fx<W>::kWidth);
     const float inv_fx = 1.f / fxs;
     const bool has_dl = a.dl != nullptr, has_iso = a.iso != nullptr;
     const int ct = threadIdx.x - 32, nct = blockDim.x - 32;
     const int cw = warp - 1;
+    unsigned* my_tile = tile + (lane & (a.copies - 1)) * a.copy_words;
     int buf = 0;            // ring slot of the next chunk (chunks consumed mod S)
     uint32_t par = 0;       // phase parity of its "full" barrier
     unsigned counted = 0;
@@ -836,8 +872,8 @@ __device__ __forceinline__ void scatter_body(const ScatterArgs& a) {
                 bad = true;
                 break;
             }
-            counted += scatter_chunk<Acc>(a, stage_view(smem + buf * sb, ch, has_dl, has_iso), min(ch, b - cs),
-                                          k_start, tk, tile, fxs, ct, nct);
+            counted += scatter_chunk<W>(a, stage_view(smem + buf * sb, ch, has_dl, has_iso), min(ch, b - cs),
+                                        k_start, tk, my_tile, fxs, ct, nct);
             __syncwarp();
             if (lane == 0) mbar_arrive(&empty[buf]);   // this warp is done with the buffer
             if (++buf == S) {
@@ -857,8 +893,12 @@ __device__ __forceinline__ void scatter_body(const ScatterArgs& a) {
             if (threadIdx.x == 32) atomicExch(a.err, 1u);
             return;
         }
+        if (a.copies > 1) {
+            fold_copies<W>(a, tile, ct, nct);
+            asm volatile("bar.sync 1, %0;" ::"r"(nct) : "memory");
+        }
         if (proj_tc) {
-            if constexpr (sizeof(Acc) == 4) {
+            if constexpr (!W) {
                 if (a.proj_nr == 2)
                     flush_tc<2, U>(a, tile, frag_s, offs_s, k_start, tk, inv_fx, cw, n_cons_warps, lane);
                 else
@@ -876,15 +916,15 @@ __device__ __forceinline__ void scatter_body(const ScatterArgs& a) {
                 const int cg = t % ncg, rb = t / ncg;
                 const int c = (cg << 6) + lane;
                 if (c >= tk) continue;
-                const Acc* col = tile + c;
+                const unsigned* col = tile + c;
                 const float4* cf = reinterpret_cast<const float4*>(coef) + rb;
                 const int cstep = a.proj_rp >> 2;
                 const bool two = c + 32 < tk;
                 float y0 = 0.f, y1 = 0.f, y2 = 0.f, y3 = 0.f, z0 = 0.f, z1 = 0.f, z2 = 0.f, z3 = 0.f;
 #pragma unroll 4
                 for (int nd = 0; nd < a.n_real; ++nd) {
-                    const float v = Fx<Acc>::to_float(col[nd * pitch]);
-                    const float u = two ? Fx<Acc>::to_float(col[nd * pitch + 32]) : 0.f;
+                    const float v = Fx<W>::value(col + nd * pitch, hi_off);
+                    const float u = two ? Fx<W>::value(col + nd * pitch + 32, hi_off) : 0.f;
                     const float4 w = cf[nd * cstep];
                     y0 = fmaf(w.x, v, y0);
                     y1 = fmaf(w.y, v, y1);
@@ -912,14 +952,17 @@ __device__ __forceinline__ void scatter_body(const ScatterArgs& a) {
             // two: exact scaling of the rounded word), with plain stores (this
             // CTA owns its columns), and re-zero it
             for (int node = cw; node < a.n_nodes; node += n_cons_warps) {
-                Acc* row = tile + node * pitch;
+                unsigned* row = tile + node * pitch;
                 float* dst = a.ldm + node * a.row_stride + k_start;
                 for (int c = lane; c < tk; c += 32) {   // one 128-byte store per warp step
                     // streaming store: the LDM is read once by the next stage, long after
-                    __stcs(&dst[c], Fx<Acc>::to_float(row[c]) * inv_fx);
+                    __stcs(&dst[c], Fx<W>::value(row + c, hi_off) * inv_fx);
                     row[c] = 0;
+                    if constexpr (W) row[hi_off + c] = 0;
                 }
             }
+            if (a.copies > 1)   // the other copies
+                zero_tile(tile + a.copy_words, n_words - a.copy_words, ct, nct);
         }
         asm volatile("bar.sync 1, %0;" ::"r"(nct) : "memory");
     }
@@ -929,9 +972,9 @@ __device__ __forceinline__ void scatter_body(const ScatterArgs& a) {
     }
 }
 
-template <typename Acc>
+template <bool W>
 __global__ void __launch_bounds__(kScatThreads, 1) k_scatter(const ScatterArgs a) {
-    scatter_body<Acc>(a);
+    scatter_body<W>(a);
 }
 
 // The accumulator chosen on the device from the column bound *cmax (served and
@@ -941,9 +984,9 @@ __global__ void __launch_bounds__(kScatThreads, 1) k_scatter(const ScatterArgs a
 // variant only take fewer tiles each).
 __global__ void __launch_bounds__(kScatThreads, 1) k_scatter_auto(const ScatterArgs a32, const ScatterArgs a64) {
     if (fx_wide(*a32.cmax))
-        scatter_body<unsigned long long, 1>(a64);
+        scatter_body<true, 1>(a64);
     else
-        scatter_body<unsigned, 1>(a32);
+        scatter_body<false, 1>(a32);
 }
 
 // ---------------------------------------------------------------------------
@@ -1999,11 +2042,11 @@ int launch_col_cmax(const int64_t* col_start, int col_off, int col_count, int n_
 
 int launch_scatter(const ScatterArgs& a, int grid, int threads, size_t smem, bool wide, cudaStream_t st) {
     if (wide) {
-        ALLOW_SMEM(k_scatter<unsigned long long>, smem);
-        k_scatter<unsigned long long><<<grid, threads, smem, st>>>(a);
+        ALLOW_SMEM(k_scatter<true>, smem);
+        k_scatter<true><<<grid, threads, smem, st>>>(a);
     } else {
-        ALLOW_SMEM(k_scatter<unsigned>, smem);
-        k_scatter<unsigned><<<grid, threads, smem, st>>>(a);
+        ALLOW_SMEM(k_scatter<false>, smem);
+        k_scatter<false><<<grid, threads, smem, st>>>(a);
     }
     return check_launch();
 }
@@ -2016,7 +2059,7 @@ int launch_scatter_auto(const ScatterArgs& a32, const ScatterArgs& a64, int grid
 }
 
 // Dynamic shared memory a scatter variant may have (one CTA per SM).
-template <typename Acc>
+template <bool W>
 static int scatter_optin(size_t* avail) {
     static std::atomic<size_t> cached{0};   // one GPU model per process
     size_t a = cached.load();
@@ -2026,7 +2069,7 @@ static int scatter_optin(size_t* avail) {
         if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess)
             return RG_ERR_CUDA;
         cudaFuncAttributes fa;
-        if (cudaFuncGetAttributes(&fa, k_scatter<Acc>) != cudaSuccess) return RG_ERR_CUDA;
+        if (cudaFuncGetAttributes(&fa, k_scatter<W>) != cudaSuccess) return RG_ERR_CUDA;
         a = (size_t)optin - fa.sharedSizeBytes;
         cached.store(a);
     }
@@ -2036,7 +2079,7 @@ static int scatter_optin(size_t* avail) {
 int scatter_smem_optin(size_t* avail, bool wide) {
     // every variant (and k_scatter_auto) has the same static shared memory
     // (none); the opt-in limit of one serves for all
-    return wide ? scatter_optin<unsigned long long>(avail) : scatter_optin<unsigned>(avail);
+    return wide ? scatter_optin<true>(avail) : scatter_optin<false>(avail);
 }
 
 template <int N1>

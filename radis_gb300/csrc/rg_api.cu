@@ -2251,7 +2251,7 @@ int rg_slit_convolve(rg_ctx* ctx, const float* in_dev, int64_t n, const float* s
     a.m = n_slit;
     a.scale = (float)wstep;
     a.valid = mode == RG_SLIT_VALID;
-    RG(launch_slit_conv(a, st));
+    RG(launch_slit_conv(a, ctx->sms, st));
     return RG_OK;
 }
 

@@ -452,7 +452,7 @@ int launch_node_project(const ProjArgs& a, cudaStream_t st);
 // would exceed r_max (rg_skeleton.cpp)
 int interp_decomp(const double* A, int S, int n, double tol, int r_max, int* sk, double* C, int* R_out,
                   double* err_out);
-int launch_slit_conv(const SlitArgs& a, cudaStream_t st);
+int launch_slit_conv(const SlitArgs& a, int sms, cudaStream_t st);
 int launch_scatter_tangent(const GradArgs& a, int grid, cudaStream_t st);
 int col_block(int n1);               // columns per CTA of the column FFTs
 int row_threads(const FftLen& f);    // block size of the forward row kernel

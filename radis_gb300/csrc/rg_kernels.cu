@@ -1714,18 +1714,29 @@ __global__ void __launch_bounds__(256) k_gauss_merge(const GaussArgs a) {
 // out[i] = scale sum_j slit[j] in[i + (m-1)/2 - j], the 'same' part of the
 // full convolution, zero outside [0, n); written as a correlation with the
 // reversed slit r[u] = slit[m-1-u]: out[i] = scale sum_u r[u] in[i - m/2 + u].
-// One CTA: kGaussTile outputs (8 per thread); taps in passes of kSlitPass,
-// each with its own staged input window, through the same register-window
-// convolution as the Gaussian stage.  'valid' mode: the first (la-1)/2 and
-// last la/2 outputs are NaN, la = min(n, m).
-__global__ void __launch_bounds__(256) k_slit_conv(const SlitArgs a) {
+// One CTA: two groups of threads over the same outputs, 8 per thread, each
+// with half of the taps (their parts are summed at the end); taps in passes of
+// kSlitPass with a staged input window, through the same register-window
+// convolution as the Gaussian stage.  'valid' mode: the first (la-1)/2 and last
+// la/2 outputs are NaN, la = min(n, m).  Bound by the FP32 pipe and its
+// operand reads (84% of the instructions are FMAs of three registers, which
+// measured 3.2 of 4 per cycle), so every SM gets the same number of outputs
+// (slit_threads) and the second group keeps enough warps in flight.  400 001
+// points x 1001 taps, time per call: 196 CTAs of 2048 outputs 28.7 us, equal
+// CTAs 26.7, with two groups 22.6 (three 22.5, four 28.2: registers allow one
+// CTA less).  A padded window without bank conflicts: 24.6.
+constexpr int kSlitGroups = 2;
+__global__ void __launch_bounds__(128 * kSlitGroups) k_slit_conv(const SlitArgs a) {
     extern __shared__ __align__(16) float ssm[];
-    constexpr int TW = kGaussTile;
     constexpr int P = kGaussPer;
+    constexpr int G = kSlitGroups;
+    const int T = (int)blockDim.x / G;       // threads of a group
+    const int TW = T * P;
+    const int grp = threadIdx.x / T, gt = threadIdx.x - grp * T;
     float* taps = ssm;                       // kSlitPass (padded to 4)
     float* xs = ssm + kSlitPass + 16;        // TW + KP + 8 <= TW + kSlitPass + 16
     const int64_t p0 = (int64_t)blockIdx.x * TW;
-    const int t0 = threadIdx.x * P;
+    const int t0 = gt * P;
     const int64_t half = a.m / 2;
     float acc[P];
 #pragma unroll
@@ -1741,7 +1752,23 @@ __global__ void __launch_bounds__(256) k_slit_conv(const SlitArgs a) {
             xs[t] = k >= 0 && k < a.n ? __ldg(&a.in[k]) : 0.f;
         }
         __syncthreads();
-        conv_window(acc, xs, taps, t0, KP);
+        // this group's share of the pass's taps
+        const int share = ((KP + G - 1) / G + 7) & ~7;
+        const int k0 = min(grp * share, KP), k1 = min(k0 + share, KP);
+        conv_window(acc, xs, taps + k0, t0 + k0, k1 - k0);
+    }
+    if (G > 1) {   // sum the groups' parts into the first one's
+        __syncthreads();
+        float* part = xs;   // [G - 1][P][T]
+        if (grp) {
+#pragma unroll
+            for (int i = 0; i < P; ++i) part[((grp - 1) * P + i) * T + gt] = acc[i];
+        }
+        __syncthreads();
+        if (grp) return;
+        for (int q = 0; q < G - 1; ++q)
+#pragma unroll
+            for (int i = 0; i < P; ++i) acc[i] += part[(q * P + i) * T + gt];
     }
     const int64_t la = a.n < (int64_t)a.m ? a.n : (int64_t)a.m;
     const int64_t ea = a.valid ? (la - 1) / 2 : 0, eb = a.valid ? la / 2 : 0;
@@ -2395,13 +2422,25 @@ int launch_gauss_merge(const GaussArgs& a0, int out_rows, cudaStream_t st) {
     return check_launch();
 }
 
-int launch_slit_conv(const SlitArgs& a, cudaStream_t st) {
+// Threads per group of the slit convolution: the outputs dealt out in the
+// fewest whole CTAs per SM of at most 128 threads a group, all equally large,
+// so that no SM works while the others have finished.
+static int slit_threads(int64_t n, int sms) {
+    const int64_t per_sm = (n + (int64_t)sms * kGaussPer - 1) / ((int64_t)sms * kGaussPer);   // threads
+    const int64_t ctas = (per_sm + 127) / 128;
+    return (int)std::max<int64_t>(8, (per_sm + ctas - 1) / ctas);
+}
+
+int launch_slit_conv(const SlitArgs& a, int sms, cudaStream_t st) {
     if (a.n <= 0) return RG_OK;
     if (a.m <= 0) return RG_ERR_RANGE;
-    const size_t smem = sizeof(float) * ((kSlitPass + 16) + (kGaussTile + kSlitPass + 16));
-    const int64_t blocks = (a.n + kGaussTile - 1) / kGaussTile;
+    const int threads = slit_threads(a.n, sms);
+    const int tile = threads * kGaussPer;
+    const size_t window = std::max(tile + kSlitPass + 16, (kSlitGroups - 1) * tile);
+    const size_t smem = sizeof(float) * (kSlitPass + 16 + window);
+    const int64_t blocks = (a.n + tile - 1) / tile;
     if (blocks > 0x7fffffff) return RG_ERR_RANGE;
-    k_slit_conv<<<(unsigned)blocks, 256, smem, st>>>(a);
+    k_slit_conv<<<(unsigned)blocks, threads * kSlitGroups, smem, st>>>(a);
     return check_launch();
 }
 

@@ -402,21 +402,95 @@ __global__ void k_prepare_lines(const double* __restrict__ v0, const double* __r
     if (i + 1 < n && v0[i + 1] < v) atomicExch(unsorted, 1);
 }
 
-// first line index with v0 >= vmin + c dv, for c = c_min + idx
-__global__ void k_col_index(const float2* __restrict__ v0, int64_t n, double vmin, double dv, int c_min,
-                            int count, int64_t* __restrict__ col_start) {
-    int idx = blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= count) return;
-    const double target = vmin + (double)(c_min + idx) * dv;
-    int64_t lo = 0, hi = n;
+// A position as v0 is stored (hi rounded to nearest, lo the rest) and the
+// comparison "v0 < target" in FP32: hi decides unless equal, then lo against
+// the rest of the target rounded up (exact for a float lo).  FP64 adds and
+// compares would bound the searches (2 lanes per clock and SM on this part).
+struct SplitTarget {
+    float hi, lo;
+};
+__device__ __forceinline__ SplitTarget split_target(double t) {
+    SplitTarget s;
+    s.hi = __double2float_rn(t);
+    s.lo = __double2float_ru(t - (double)s.hi);
+    return s;
+}
+__device__ __forceinline__ bool below(float2 w, SplitTarget t) { return w.x < t.hi || (w.x == t.hi && w.y < t.lo); }
+
+// First line index with v0 >= target, by one warp: 32 pivots per step, so a list
+// of 10M lines takes 5 dependent loads instead of 24.
+__device__ __forceinline__ int64_t warp_lower_bound(const float2* __restrict__ v0, int64_t n, SplitTarget target,
+                                                    int lane) {
+    int64_t lo = 0, hi = n;   // the answer lies in [lo, hi]
     while (lo < hi) {
-        int64_t mid = lo + ((hi - lo) >> 1);
-        float2 w = v0[mid];
-        double v = (double)w.x + (double)w.y;
-        if (v < target)
-            lo = mid + 1;
-        else
-            hi = mid;
+        // pivots lo <= p_0 <= ... <= p_31 < hi; v0 ascends, so the lanes below the target come first
+        const int64_t p = lo + ((hi - lo) * lane >> 5);
+        const int nb = __popc(__ballot_sync(0xffffffffu, below(v0[p], target)));
+        const int64_t a = lo + ((hi - lo) * (nb - 1) >> 5), b = lo + ((hi - lo) * nb >> 5);
+        if (nb == 0) return lo;
+        if (nb < 32) hi = b;
+        lo = a + 1;
+    }
+    return lo;
+}
+
+// First line index with v0 >= vmin + c dv, for c = c_min + idx.  Bound by the
+// latency of dependent loads: a block finds the lines between its first and
+// last column with two warps (above), and its threads search between them, in
+// shared memory when they are few enough.  (One binary search of the whole
+// list per column, compared in FP64: 76 us on 5M lines x 400 001 columns, 20 us on
+// 600k lines x 116k columns, alone on a cold GPU; now 25 and 9.)
+constexpr int kColStage = 2048;
+__global__ void __launch_bounds__(256) k_col_index(const float2* __restrict__ v0, int64_t n, double vmin, double dv,
+                                                   int c_min, int count, int64_t* __restrict__ col_start) {
+    __shared__ int64_t ends[2];
+    __shared__ float2 part[kColStage];
+    const int idx = blockIdx.x * 256 + threadIdx.x;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    auto target_of = [&](int i) { return split_target(vmin + (double)(c_min + i) * dv); };
+    if (warp < 2) {
+        const int i = min((int)blockIdx.x * 256 + (warp ? 255 : 0), count - 1);
+        const int64_t b = warp_lower_bound(v0, n, target_of(i), lane);
+        if (lane == 0) ends[warp] = b;
+    }
+    __syncthreads();
+    const int64_t first = ends[0];
+    const int m = (int)min(ends[1] - first, (int64_t)0x7fffffff);
+    const bool staged = m <= kColStage;
+    if (staged) {
+        for (int i = threadIdx.x; i < m; i += 256) part[i] = v0[first + i];
+        __syncthreads();
+    }
+    if (idx >= count) return;
+    const SplitTarget target = target_of(idx);
+    int64_t lo = first, hi = ends[1];
+    if (staged) {
+        int l = 0, h = m;
+        while (l < h) {
+            const int mid = (l + h) >> 1;
+            if (below(part[mid], target))
+                l = mid + 1;
+            else
+                h = mid;
+        }
+        lo = first + l;
+    } else {
+        while (lo < hi) {   // eight parts per step: seven independent loads
+            const int64_t span = hi - lo;
+            int nb = 0;
+#pragma unroll
+            for (int i = 1; i < 8; ++i) nb += below(v0[lo + (span * i >> 3)], target);
+            const int64_t a = lo + (span * nb >> 3), b = lo + (span * (nb + 1) >> 3);
+            if (nb < 7) hi = b;   // v0[b] is not below the target
+            if (nb > 0)
+                lo = a + 1;          // v0[a] is
+            else if (span < 8) {     // the first part may be empty: look at lo itself
+                if (below(v0[lo], target))
+                    ++lo;
+                else
+                    hi = lo;
+            }
+        }
     }
     col_start[idx] = lo;
 }

@@ -143,7 +143,8 @@ typedef struct {
     double log_wL_min, dxL;
     int n_G, n_L;
     int64_t n_ft;              /* FFT length                                   */
-    int64_t n1, n2;            /* FFT factorisation n_ft = n1 * n2             */
+    int64_t n1, n2;            /* the form n_ft = n1 * n2 of the length (the
+                                  kernels split it as they like)               */
 } rg_grid;
 
 typedef struct {

@@ -149,8 +149,9 @@ struct Work {
     rg_plan_desc desc{};
     // FFT factorisation n = n1 n2 and its tables
     int64_t n = 0;
-    int n1 = 0, n2 = 0, B = 0;
-    FftLen f1, f2;
+    int n1 = 0, n2 = 0;
+    int form1 = 0, form2 = 0;         // the length's form that rg_grid reports (choose_fft)
+    FftLen f2;
     const float2* tw_hi = nullptr;
     const float2* tw_lo = nullptr;
     // line index per grid column and the fixed-point bound
@@ -196,8 +197,8 @@ struct Work {
     int last_accum = 0;               // accumulator bits of the last scatter (0: chosen on the device)
     int64_t row_stride = 0;
     float* ldm = nullptr;             // LDM [node][row_stride] (the scatter's float values)
-    float2* y = nullptr;
-    float2* g = nullptr;
+    float4* y = nullptr;              // [pair][n1][n2 / 2] (rg_fft.cu)
+    float4* g = nullptr;              // [n1][n2 / 2]
     unsigned long long* counter = nullptr;
     unsigned* err = nullptr;          // device flag set by a bounded wait that gave up
     unsigned* err_host = nullptr;     // pinned copy of err, refreshed after every spectrum
@@ -253,10 +254,6 @@ int64_t next_smooth(int64_t x) {
     }
 }
 
-// Radix plan of a length L = 2^a 3^b 5^c: the leftover 2 or 4, the 3s and 5s
-// (merged into composite radices: up to 12 first, 6 later), then radix 8
-// -- the last pass is radix 8 whenever 8 divides L, which the row kernel
-// relies on (n2 is a multiple of 32).
 // Partition-function ratio Q(Tref)/Q(T) of isotopologue i: the caller's,
 // else the list's tables when every isotopologue has one, else 1.
 bool have_qtables(const rg_lines* L) {
@@ -293,62 +290,75 @@ int dlnq_of(const rg_lines* L, const double* dlnq_dT, double T, int i, double* o
     return RG_OK;
 }
 
-bool radices(int L, int* rad, int* np) {
-    int r = L, k = 0;
-    int a = 0, b = 0, c = 0;
-    while (r % 2 == 0) {
-        r /= 2;
-        ++a;
-    }
-    while (r % 3 == 0) {
-        r /= 3;
-        ++b;
-    }
-    while (r % 5 == 0) {
-        r /= 5;
-        ++c;
-    }
-    // the small factors (the leftover 2 or 4, the 3s and 5s), merged in order
-    // into composite radices (6, 9, 10, 12) within the bounds the row kernels
-    // transform in registers without spilling
-    int small[64], ns = 0;
-    if (a % 3 == 2) small[ns++] = 4;
-    if (a % 3 == 1) small[ns++] = 2;
-    for (int i = 0; i < b && ns < 64; ++i) small[ns++] = 3;
-    for (int i = 0; i < c && ns < 64; ++i) small[ns++] = 5;
-    int cur = 1;
-    for (int i = 0; i < ns; ++i) {
-        const int cap = k == 0 ? kFirstRadixMax : kMidRadixMax;
-        if (cur * small[i] <= cap) {
-            cur *= small[i];
-        } else {
-            if (k >= kMaxPasses) return false;
-            rad[k++] = cur;
-            cur = small[i];
+// Radix plan of a row DFT's packed length h = 2^a 3^b 5^c (>= 16): the fewest
+// passes (each costs a trip through shared memory and a barrier), then the
+// least arithmetic.  `cost`: packed instructions per point of a radix's
+// butterfly with its twiddles.
+bool radices(int h, int* rad, int* np) {
+    struct Radix {
+        int r;
+        double dft, tw;
+    };
+    static const Radix all[] = {{12, 8.7, 6.0}, {10, 8.4, 5.8}, {9, 9.3, 5.8}, {8, 6.5, 5.5}, {6, 7.3, 5.4},
+                                {5, 6.4, 4.8},  {4, 4.0, 4.0},  {3, 4.0, 3.4}, {2, 2.0, 2.5}};
+    int best[kMaxPasses], cur[kMaxPasses], nbest = kMaxPasses + 1;
+    double cbest = 0.0;
+    auto go = [&](auto&& self, int rest, int k, double c) -> void {
+        if (rest == 1) {
+            if (k >= 2 && (k < nbest || (k == nbest && c < cbest))) {
+                nbest = k;
+                cbest = c;
+                std::copy(cur, cur + k, best);
+            }
+            return;
         }
-    }
-    if (cur > 1) {
-        if (k >= kMaxPasses) return false;
-        rad[k++] = cur;
-    }
-    for (int i = 0; i < a / 3; ++i) {
-        if (k >= kMaxPasses) return false;
-        rad[k++] = 8;
-    }
-    *np = k;
-    return r == 1;
+        if (k >= std::min(nbest, kMaxPasses)) return;
+        for (const Radix& x : all) {
+            if (rest % x.r || x.r > (k ? kMidRadixMax : kFirstRadixMax)) continue;
+            if (k >= 2 && x.r > cur[k - 1]) continue;   // later radices descend: each set once
+            cur[k] = x.r;
+            self(self, rest / x.r, k + 1, c + x.dft + (k ? x.tw : 0.0));
+        }
+    };
+    go(go, h, 0, 0.0);
+    if (nbest > kMaxPasses) return false;
+    *np = nbest;
+    std::copy(best, best + nbest, rad);
+    return true;
 }
 
-constexpr int kN2Max = 256 * 32;   // row FFT limit (threads x register accumulators)
+constexpr int kN2Max = 256 * 32;   // row FFT limit (two shared buffers of n2 / 2 elements)
 
-// choose n = n1 * n2 >= n_min, n1 a power of two <= 512, n2 = 32 * (5-smooth).
-// The row kernel runs n1 x (pair groups) CTAs, so n1 = 8 (a handful of long
-// rows) is taken only when its length is at least a quarter shorter than the
-// best with n1 = 512 or 64, or when neither fits.
+// Factorisation of a transform length n into n1 rows (column DFTs of length
+// n1) of n2 points, n2 a multiple of 8.  Rows run one per CTA, so n1 is at least
+// 256 where n2 stays >= 32; longer columns cost a shared-memory exchange more
+// (512: two, 1024: three) and rows shorter than ~2400 points gain nothing.  Column + row
+// + inverse column stage on GB300 (us, stage events): 40 960 points 29.6 (64
+// rows), 28.5 (128), 26.6 (256), 28.5 (512); 245 760 points 48.6, 36.6, 33.4,
+// 34.7; 307 200: 61.3, 39.6, 37.4, 36.8; 819 200: 73.4 (256), 66.5 (512), 72.6
+// (1024); 3 145 728: 478 (512), 445 (1024).
+void split_fft(int64_t n, int* n1o, int* n2o) {
+    const int want = n <= 300000 ? 256 : n <= 2000000 ? 512 : 1024;
+    int best = 0;
+    for (int n1 = 8; n1 <= 1024; n1 *= 2) {
+        if (n % n1) continue;
+        const int64_t n2 = n / n1;
+        if (n2 % 8 || n2 > kN2Max || n2 < 32) continue;
+        if (!best || n1 <= want) best = n1;   // the largest up to `want`, else the smallest
+    }
+    *n1o = best;
+    *n2o = (int)(n / best);
+}
+
+// The transform length n >= n_min: the shortest n1' n2' with n1' in {512, 64,
+// 8} and n2' = 32 x (5-smooth) <= kN2Max (n1' = 8 only when it is at least a
+// quarter shorter than the best of the others, or when neither fits), or
+// `forced` if it has such a form.  n1', n2' are what rg_grid reports; the
+// kernels split the length themselves (split_fft).
 bool choose_fft(int64_t n_min, int64_t forced, int* n1o, int* n2o) {
     int64_t best = std::numeric_limits<int64_t>::max();
-    int b1 = 0, b2 = 0;
-    for (int n1 : {512, 64, 8}) {   // radix-8 register column FFTs
+    bool any = false;
+    for (int n1 : {512, 64, 8}) {
         int64_t n2;
         if (forced) {
             if (forced % n1) continue;
@@ -365,18 +375,15 @@ bool choose_fft(int64_t n_min, int64_t forced, int* n1o, int* n2o) {
         if (n2 > kN2Max) continue;
         int64_t n = (int64_t)n1 * n2;
         if (n < n_min) continue;
-        // prefer the shorter transform, then the larger n1 (fewer row FFT launches)
-        if (n1 == 8 && !forced && b1 && 4 * n > 3 * best) continue;
+        if (n1 == 8 && !forced && any && 4 * n > 3 * best) continue;
         if (n < best) {
             best = n;
-            b1 = n1;
-            b2 = (int)n2;
+            any = true;
+            *n1o = n1;
+            *n2o = (int)n2;
         }
     }
-    if (!b1) return false;
-    *n1o = b1;
-    *n2o = b2;
-    return true;
+    return any;
 }
 
 int upload_twiddles(int L, float2** out) {
@@ -391,16 +398,26 @@ int upload_twiddles(int L, float2** out) {
     return RG_OK;
 }
 
-int make_fftlen(int L, FftLen* f) {
-    f->L = L;
-    if (!radices(L, f->radix, &f->npass)) return fail(RG_ERR_RANGE, "FFT length %d not factorable", L);
+// Row plan of n2 points (without its table) and the tables of both lengths.
+int row_plan(int n2, FftLen* f) {
+    auto magic = [](int d) { return (unsigned)(((1ull << 32) + d - 1) / (unsigned long long)d); };
+    f->L = n2 / 2;
+    if (!radices(f->L, f->radix, &f->npass)) return fail(RG_ERR_RANGE, "FFT length %d not factorable", n2);
     int ns = 1;
     for (int p = 0; p < f->npass; ++p) {
         f->ns[p] = ns;
-        f->mag[p] = ns == 1 ? 0u : (unsigned)(((1ull << 32) + ns - 1) / (unsigned long long)ns);
+        f->mag[p] = ns == 1 ? 0u : magic(ns);
+        f->mag_m[p] = magic(f->L / f->radix[p]);
         ns *= f->radix[p];
     }
-    return upload_twiddles(L, &f->tw);
+    const int r0 = f->radix[0];
+    f->pad_mag = r0 % 2 ? 0u : magic(r0);
+    f->row_len = f->L + (r0 % 2 ? 0 : f->L / r0);
+    return RG_OK;
+}
+int make_row_fft(int n2, FftLen* f) {
+    RG(row_plan(n2, f));
+    return upload_twiddles(n2, &f->tw);
 }
 
 void split(double v, float* hi, float* lo) {
@@ -517,7 +534,7 @@ int compute_grid_env(const Envelope& E, const rg_lines* lines, const rg_plan_des
 }
 
 int compute_grid(const rg_lines* L, const Work& W, const rg_conditions* c, SpecHost* s) {
-    return compute_grid_env(L->env, L, W.desc, W.n, W.n1, W.n2, c, s);
+    return compute_grid_env(L->env, L, W.desc, W.n, W.form1, W.form2, c, s);
 }
 
 // Envelope of a host line list (per-iso v0 range, width and intensity hulls).
@@ -853,10 +870,7 @@ void node_fold(double dv, double wG, double wL, double thresh, int* nfold, doubl
 void fill_voigt_args(Work& W, const SpecHost& s, VoigtArgs* va) {
     const rg_grid& g = s.grid;
     va->f2 = W.f2;
-    va->threads = row_threads(W.f2);
-    const RowLayout rl = row_layout(W.n2);
-    va->pairs_per_pass = rl.pairs;
-    va->row_twiddle_table = rl.twr;
+    va->bins = 0;
     va->n1 = W.n1;
     va->n2 = W.n2;
     va->n = W.n;
@@ -865,8 +879,6 @@ void fill_voigt_args(Work& W, const SpecHost& s, VoigtArgs* va) {
     va->NL = g.n_L;
     va->y = W.y;
     va->g = W.g;
-    va->tw_hi = W.tw_hi;
-    va->tw_lo = W.tw_lo;
     va->inv_ndv = (float)(1.0 / ((double)W.n * W.desc.dv));
     va->half_fs = (float)(0.5 / W.desc.dv);
     const double thresh = W.desc.folding_thresh > 0 ? W.desc.folding_thresh : 1e-6;
@@ -914,6 +926,13 @@ void fill_voigt_args(Work& W, const SpecHost& s, VoigtArgs* va) {
     W.va_nfold.assign(va->nfold, va->nfold + s.n_nodes);
     W.va_any_fold = va->any_fold;
     W.va_valid = true;
+}
+
+// Launch shape of the row kernels for the pairs in *va.
+void set_row_shape(const Work& W, int sms, VoigtArgs* va, bool adjoint = false) {
+    const RowShape rs = row_shape(W.f2, W.n1, va->n_pairs, sms, adjoint);
+    va->units = rs.units;
+    va->threads = rs.threads;
 }
 
 // Merged layout of one spectrum.  Without folding, the Voigt FT of node
@@ -1404,17 +1423,14 @@ int enqueue_spectrum(const rg_lines* L, Work& W, const rg_conditions* c, const S
     if (!ldm_only) {
         ColFftArgs ca;
         std::memset(&ca, 0, sizeof ca);
-        ca.f1 = W.f1;
         ca.n1 = W.n1;
         ca.n2 = W.n2;
-        ca.B = W.B;
         ca.n_v = n_v;
         ca.n = W.n;
         ca.row_stride = W.row_stride;
         ca.n_pairs = s.n_nodes / 2;
         ca.ldm = W.ldm;
         ca.cmax = W.cmax_dev;
-        ca.twiddle = !row_layout(W.n2).twr;
         ca.y = W.y;
         ca.tw_hi = W.tw_hi;
         ca.tw_lo = W.tw_lo;
@@ -1467,25 +1483,13 @@ int enqueue_spectrum(const rg_lines* L, Work& W, const rg_conditions* c, const S
         }
         if (ev) CU(cudaEventRecord(ev[2], st));
         VoigtArgs& vr = skel ? *lp.vk : merged ? *lp.vm : *lp.va;
-        vr.store_g = vr.n_pairs <= kPairGroup;   // one pair group per row: it stores G itself
-        vr.inv_fused = vr.store_g;                // ... after its inverse row DFT
-        if (!vr.store_g) CU(cudaMemsetAsync(W.g, 0, sizeof(float2) * (size_t)W.n, st));
-        RG(launch_row_fft_voigt(vr, st));
+        set_row_shape(W, L->ctx->sms, &vr);
+        RG(launch_row_fft_voigt(vr, st));   // with the inverse row DFT
         if (ev) CU(cudaEventRecord(ev[3], st));
-        if (!vr.inv_fused) {
-            RowIfftArgs ra;
-            ra.f2 = W.f2;
-            ra.n1 = W.n1;
-            ra.n2 = W.n2;
-            ra.n = W.n;
-            ra.g = W.g;
-            ra.tw_hi = W.tw_hi;
-            ra.tw_lo = W.tw_lo;
-            RG(launch_row_ifft(ra, st));
-        }
         if (ev) CU(cudaEventRecord(ev[4], st));
         ca.h = W.g;
         ca.out = out;
+        ca.out_vec = (reinterpret_cast<uintptr_t>(out) & 7) == 0;
         ca.out_scale = (float)(std::exp(s.log_scale_int - s.log_scale_out) / ((double)W.n * W.desc.dv));
         ca.err = W.err;
         ca.err_pub = W.err_pub;   // mapped: the kernel publishes and clears the flag
@@ -1537,17 +1541,14 @@ int fill_grad_args(const rg_lines* L, const Work& W, const rg_conditions* c, con
 ColFftArgs col_args(const Work& W, const SpecHost& s) {
     ColFftArgs ca;
     std::memset(&ca, 0, sizeof ca);
-    ca.f1 = W.f1;
     ca.n1 = W.n1;
     ca.n2 = W.n2;
-    ca.B = W.B;
     ca.n_v = (int)W.desc.n_v;
     ca.n = W.n;
     ca.row_stride = W.row_stride;
     ca.n_pairs = s.n_nodes / 2;
     ca.tw_hi = W.tw_hi;
     ca.tw_lo = W.tw_lo;
-    ca.twiddle = !row_layout(W.n2).twr;
     return ca;
 }
 
@@ -1584,7 +1585,8 @@ int enqueue_backward(const rg_lines* L, Work& W, const rg_conditions* c, const S
     unit->lnorm[1] = -std::numeric_limits<float>::infinity();
     unit->nfold[0] = unit->nfold[1] = 0;
     unit->any_fold = 0;
-    CU(cudaMemsetAsync(W.g, 0, sizeof(float2) * (size_t)W.n, st));
+    unit->bins = 1;   // Ghat itself, no inverse
+    set_row_shape(W, L->ctx->sms, unit);
     RG(launch_row_fft_voigt(*unit, st));
     // adjoint LDM rows: Re / Im of IFFT(Ghat (V_a + i V_b)) / (N dv), per pair;
     // with the skeleton layout only the skeleton rows (the gather expands them
@@ -1598,6 +1600,7 @@ int enqueue_backward(const rg_lines* L, Work& W, const rg_conditions* c, const S
         ar->v.g = ghat.g;
     }
     ar->y = W.y;
+    set_row_shape(W, L->ctx->sms, &ar->v, true);
     RG(launch_row_ifft_adj(*ar, st));
     ColFftArgs cb = col_args(W, s);
     if (skel) cb.n_pairs = lp.pa.rows / 2;
@@ -1634,8 +1637,7 @@ int enqueue_tangent(const rg_lines* L, Work& W, const rg_conditions* c, const Sp
     LayoutPlan lp;
     const bool skel = W.desc.layout != 1 && W.desc.layout != 2 && plan_layout(W, s, st, &lp) == RG_OK && lp.skel;
     VoigtArgs& vr = skel ? *lp.vk : *va;
-    vr.store_g = vr.n_pairs <= kPairGroup;
-    vr.inv_fused = vr.store_g;
+    set_row_shape(W, L->ctx->sms, &vr);
     float* tan = W.ldm;
     ga->tan = tan;
     const int n_v = (int)W.desc.n_v;
@@ -1651,22 +1653,13 @@ int enqueue_tangent(const rg_lines* L, Work& W, const rg_conditions* c, const Sp
             RG(launch_node_project(pa, st));
             ca.n_pairs = pa.rows / 2;
         }
-        ca.src = tan;
+        ca.ldm = tan;
         ca.y = W.y;
-        RG(launch_col_fft_fwd_f(ca, st));
-        if (!vr.store_g) CU(cudaMemsetAsync(W.g, 0, sizeof(float2) * (size_t)W.n, st));
+        RG(launch_col_fft_fwd(ca, st));
         RG(launch_row_fft_voigt(vr, st));
-        RowIfftArgs ra;
-        ra.f2 = W.f2;
-        ra.n1 = W.n1;
-        ra.n2 = W.n2;
-        ra.n = W.n;
-        ra.g = W.g;
-        ra.tw_hi = W.tw_hi;
-        ra.tw_lo = W.tw_lo;
-        if (!vr.inv_fused) RG(launch_row_ifft(ra, st));
         ca.h = W.g;
         ca.out = out + (size_t)q * n_v;
+        ca.out_vec = (reinterpret_cast<uintptr_t>(ca.out) & 7) == 0;
         ca.out_scale = (float)(std::exp(s.log_scale_int - s.log_scale_out) / ((double)W.n * W.desc.dv));
         RG(launch_col_ifft(ca, st));
     }
@@ -1979,12 +1972,11 @@ int rg_plan_create(rg_lines* L, const rg_plan_desc* d, rg_plan** out) {
     if (!choose_fft(2 * d->n_v, d->n_ft, &n1, &n2))
         return fail(RG_ERR_RANGE, "no supported FFT length >= %lld (n_ft=%lld)", (long long)(2 * d->n_v),
                     (long long)d->n_ft);
-    W.n1 = n1;
-    W.n2 = n2;
+    W.form1 = n1;
+    W.form2 = n2;
     W.n = (int64_t)n1 * n2;
-    W.B = col_block(n1);
-    RG(make_fftlen(n1, &W.f1));
-    RG(make_fftlen(n2, &W.f2));
+    split_fft(W.n, &W.n1, &W.n2);
+    RG(make_row_fft(W.n2, &W.f2));
     RG(tw_n_tables(W.n, &P->tw_hi_own, &P->tw_lo_own));
     W.tw_hi = P->tw_hi_own;
     W.tw_lo = P->tw_lo_own;
@@ -2044,7 +2036,6 @@ int rg_plan_free(rg_plan* P) {
         dev_guard_.use(P->lines->ctx->device);
         cudaStreamSynchronize(P->lines->ctx->stream);
         cudaDeviceSynchronize();
-        dfree(P->w.f1.tw);
         dfree(P->w.f2.tw);
         dfree(P->tw_hi_own);
         dfree(P->tw_lo_own);
@@ -2474,7 +2465,7 @@ struct rg_server {
     std::thread worker;
     bool stop = false;
     int64_t next_ticket = 1, completed = 0, failed = 0;
-    std::map<int, FftLen> fft;                              // worker only
+    std::map<int, FftLen> fft_row;                          // worker only
     std::map<int64_t, std::pair<float2*, float2*>> twn;     // worker only
     Clock::time_point t0 = Clock::now();
     uint32_t magic = 0x52475356;
@@ -2511,16 +2502,13 @@ void CUDART_CB slot_done_cb(void* p) {
 }
 
 int server_tables(rg_server* S, Work& W) {
-    for (int L : {W.n1, W.n2}) {
-        auto it = S->fft.find(L);
-        if (it == S->fft.end()) {
-            FftLen f;
-            RG(make_fftlen(L, &f));
-            it = S->fft.emplace(L, f).first;
-        }
-        (L == W.n1 ? W.f1 : W.f2) = it->second;
+    auto it = S->fft_row.find(W.n2);
+    if (it == S->fft_row.end()) {
+        FftLen f;
+        RG(make_row_fft(W.n2, &f));
+        it = S->fft_row.emplace(W.n2, f).first;
     }
-    if (W.n1 == W.n2) W.f2 = W.f1;
+    W.f2 = it->second;
     auto t = S->twn.find(W.n);
     if (t == S->twn.end()) {
         float2 *hi = nullptr, *lo = nullptr;
@@ -2592,10 +2580,10 @@ int start_on_slot(rg_server* S, int si, const std::shared_ptr<ServerReq>& r, con
     Work& W = sl.w;
     const rg_plan_desc& d = r->desc;
     W.desc = d;
-    W.n1 = n1;
-    W.n2 = n2;
+    W.form1 = n1;
+    W.form2 = n2;
     W.n = (int64_t)n1 * n2;
-    W.B = col_block(n1);
+    split_fft(W.n, &W.n1, &W.n2);
     RG(server_tables(S, W));
     shift_margin(r->lines, d.dv, &W.E, &W.p_atm_max);
     W.col_off = W.E;
@@ -2793,16 +2781,15 @@ int rg_server_create(rg_ctx* ctx, int slots, int64_t mem_budget, rg_server** out
         *sl.w.err_host = 0;
         CU(cudaHostGetDevicePointer((void**)&sl.w.err_pub, sl.w.err_host, 0));
     }
-    // the FFT tables of every factorisation choose_fft can pick (n1 in {8, 64,
-    // 512}, n2 = 32 x 5-smooth <= kN2Max), built before the worker starts: a
-    // request never waits for a table upload (an allocation and a blocking
-    // copy) on the worker thread
+    // the FFT tables of every length choose_fft can pick ({8, 64, 512} x 32 x
+    // 5-smooth <= kN2Max), built before the worker starts: a request never
+    // waits for a table upload (an allocation and a blocking copy) on the
+    // worker thread
     for (int64_t m = 1; 32 * m <= kN2Max; m = next_smooth(m + 1))
-        for (int n1 : {8, 64, 512}) {
+        for (int f : {8, 64, 512}) {
             Work t;
-            t.n1 = n1;
-            t.n2 = (int)(32 * m);
-            t.n = (int64_t)t.n1 * t.n2;
+            t.n = f * 32 * m;
+            split_fft(t.n, &t.n1, &t.n2);
             RG(server_tables(S, t));
         }
     ctx->lines++;   // the context stays alive while the server exists
@@ -2905,7 +2892,7 @@ int rg_server_destroy(rg_server* S) {
         if (sl.pin) cudaFreeHost(sl.pin);
         cudaStreamDestroy(sl.st);
     }
-    for (auto& kv : S->fft) dfree(kv.second.tw);
+    for (auto& kv : S->fft_row) dfree(kv.second.tw);
     for (auto& kv : S->twn) {
         dfree(kv.second.first);
         dfree(kv.second.second);
@@ -2929,7 +2916,7 @@ int rg_server_destroy(rg_server* S) {
 // every GPU that loads this library holds it until the process exits.
 constexpr size_t kStaticScratchBytes = (size_t)64 << 20;   // 64 MiB
 static __device__ __align__(256) unsigned char g_static_scratch[kStaticScratchBytes];
-constexpr size_t kStaticProjBytes = 256 * 1024;
+constexpr size_t kStaticProjBytes = 254 * 1024;
 
 namespace {
 
@@ -2950,19 +2937,6 @@ __global__ void k_static_twiddles(float2* tw, int count, long long L, long long 
 int static_twiddles(float2* tw, int count, long long L, long long stride, cudaStream_t st) {
     k_static_twiddles<<<(count + 255) / 256, 256, 0, st>>>(tw, count, L, stride);
     return cudaGetLastError() == cudaSuccess ? RG_OK : RG_ERR_CUDA;
-}
-
-// radix plan of one FFT length without any table (the table goes to scratch)
-int static_fftlen(int L, FftLen* f) {
-    f->L = L;
-    if (!radices(L, f->radix, &f->npass)) return fail(RG_ERR_RANGE, "FFT length %d not factorable", L);
-    int ns = 1;
-    for (int p = 0; p < f->npass; ++p) {
-        f->ns[p] = ns;
-        f->mag[p] = ns == 1 ? 0u : (unsigned)(((1ull << 32) + ns - 1) / (unsigned long long)ns);
-        ns *= f->radix[p];
-    }
-    return RG_OK;
 }
 
 }  // namespace
@@ -2997,18 +2971,17 @@ extern "C" int rg_synthesize_static(rg_lines* L, const rg_plan_desc* d, const rg
     int n1, n2;
     if (!choose_fft(2 * d->n_v, d->n_ft, &n1, &n2))
         return fail(RG_ERR_RANGE, "no supported FFT length >= %lld", (long long)(2 * d->n_v));
-    W.n1 = n1;
-    W.n2 = n2;
+    W.form1 = n1;
+    W.form2 = n2;
     W.n = (int64_t)n1 * n2;
-    W.B = col_block(n1);
-    RG(static_fftlen(n1, &W.f1));
-    RG(static_fftlen(n2, &W.f2));
+    split_fft(W.n, &W.n1, &W.n2);
+    RG(row_plan(W.n2, &W.f2));   // its table goes to the scratch
     shift_margin(L, d->dv, &W.E, &W.p_atm_max);
     W.col_off = W.E;
     W.col_count = (int)d->n_v + 1 + 2 * W.E;
     W.row_stride = (d->n_v + 31) / 32 * 32;
     SpecHost s;
-    RG(compute_grid_env(L->env, L, W.desc, W.n, W.n1, W.n2, c, &s));
+    RG(compute_grid_env(L->env, L, W.desc, W.n, W.form1, W.form2, c, &s));
 
     // carve the scratch (256-byte aligned pieces)
     size_t off = 0;
@@ -3022,8 +2995,7 @@ extern "C" int rg_synthesize_static(rg_lines* L, const rg_plan_desc* d, const rg
     W.cmax_dev = static_cast<int*>(take(sizeof(int)));
     W.counter = static_cast<unsigned long long*>(take(sizeof(unsigned long long)));
     W.err = static_cast<unsigned*>(take(sizeof(unsigned)));
-    W.f1.tw = static_cast<float2*>(take(sizeof(float2) * (size_t)n1));
-    W.f2.tw = static_cast<float2*>(take(sizeof(float2) * (size_t)n2));
+    W.f2.tw = static_cast<float2*>(take(sizeof(float2) * (size_t)W.n2));
     float2* twh = static_cast<float2*>(take(sizeof(float2) * (size_t)nh));
     float2* twl = static_cast<float2*>(take(sizeof(float2) * 1024));
     W.tw_hi = twh;
@@ -3040,8 +3012,8 @@ extern "C" int rg_synthesize_static(rg_lines* L, const rg_plan_desc* d, const rg
     W.ldm_bytes = sizeof(float) * (size_t)s.n_nodes * (size_t)W.row_stride;
     W.y_bytes = sizeof(float2) * (size_t)(s.n_nodes / 2) * (size_t)W.n;
     W.ldm = static_cast<float*>(take(W.ldm_bytes));
-    W.y = static_cast<float2*>(take(W.y_bytes));
-    W.g = static_cast<float2*>(take(sizeof(float2) * (size_t)W.n));
+    W.y = static_cast<float4*>(take(W.y_bytes));
+    W.g = static_cast<float4*>(take(sizeof(float2) * (size_t)W.n));
     if (off > kStaticScratchBytes)
         return fail(RG_ERR_RANGE,
                     "spectrum needs %zu bytes of scratch, more than the %zu-byte static array of the "
@@ -3062,8 +3034,7 @@ extern "C" int rg_synthesize_static(rg_lines* L, const rg_plan_desc* d, const rg
     drain.armed = true;
     // every piece starts from what the previous call left: clear what must be zero
     CU(cudaMemsetAsync(W.err, 0, sizeof(unsigned), st));
-    RG(static_twiddles(W.f1.tw, n1, n1, 1, st));
-    RG(static_twiddles(W.f2.tw, n2, n2, 1, st));
+    RG(static_twiddles(W.f2.tw, W.n2, W.n2, 1, st));
     RG(static_twiddles(twh, nh, W.n, 1024, st));
     RG(static_twiddles(twl, 1024, W.n, 1, st));
     RG(launch_col_index(L->v0, L->n, d->vmin, d->dv, -W.E, W.col_count, W.col_start, st));

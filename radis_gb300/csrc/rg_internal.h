@@ -17,6 +17,7 @@
 #include <cuda_runtime.h>
 #else
 struct float2 { float x, y; };
+struct float4 { float x, y, z, w; };
 typedef struct CUstream_st* cudaStream_t;
 #endif
 
@@ -38,14 +39,13 @@ constexpr double kAtm = 1.01325;                    // bar per atm (broadening.p
 constexpr int kMaxIso = 16;
 constexpr int kMaxAxis = 64;        // max nodes along one LDM axis
 constexpr int kMaxNodes = 1024;     // max N_G * N_L (padded to even)
-constexpr int kPairGroup = 16;      // node pairs per Voigt-reduce work item
 constexpr int kMaxPasses = 16;
-// FFT radix plans merge the small factors into composite radices of at most
-// kFirstRadixMax in the first pass (no pass twiddles) and kMidRadixMax later:
-// the bounds under which the row kernels keep two pairs' butterflies in
-// registers without spilling
+// Largest radix of the row DFTs' first pass (no pass twiddles) and of the later
+// ones: the bounds under which the row kernels keep a butterfly in registers
+// without spilling.
 constexpr int kFirstRadixMax = 12;
-constexpr int kMidRadixMax = 6;
+constexpr int kMidRadixMax = 10;
+constexpr int kRowMaxThreads = 768;   // of the row kernels' CTAs
 
 // --- host work over line arrays ------------------------------------------------
 // [0, n) in T contiguous chunks, chunk t = [n t / T, n (t + 1) / T): one per
@@ -96,13 +96,18 @@ Hull lower_hull_src(const PointSource& s);
 Hull upper_hull_src(const PointSource& s);
 
 // --- FFT plan of one sub-length -------------------------------------------------
+// Rows of n2 points: the packed passes run over L = n2 / 2 (rg_fft.cu), the
+// table has n2 entries.
 struct FftLen {
     int L = 0;
     int npass = 0;
     int radix[kMaxPasses] = {0};
     int ns[kMaxPasses] = {0};          // sub-transform length before each pass
     unsigned mag[kMaxPasses] = {0};    // ceil(2^32 / ns): j / ns == umulhi(j, mag) for j, ns < 2^16
-    float2* tw = nullptr;       // device: exp(-2 pi i t / L), t < L
+    unsigned mag_m[kMaxPasses] = {0};  // the same for L / radix
+    unsigned pad_mag = 0;              // the same for an even first radix, else 0
+    int row_len = 0;                   // elements of a transform's shared buffer
+    float2* tw = nullptr;              // device: exp(-2 pi i t / n)
 };
 
 // --- kernel argument blocks (passed by value) ----------------------------------
@@ -202,25 +207,23 @@ RG_HD inline int scatter_copy_words(int n_nodes, int pitch, bool wide, int copie
 RG_HD inline size_t scatter_coef_offset(size_t words) { return (words * 4 + 15) / 16 * 16; }
 
 struct ColFftArgs {       // K2 (forward column FFT) and K4 (inverse column FFT)
-    FftLen f1;
     int n1, n2;
-    int B;                // columns per CTA
     int n_v;
     int64_t n;            // n_ft
     int64_t row_stride;
     int n_pairs;
     const float* ldm;     // K2 input: the scatter's LDM [node][row_stride]
     const int* cmax;      // device: fixed-point bound of the scatter (scale = fx_scale(*cmax))
-    float2* y;            // K2 output [pair][n1][n2]
+    float4* y;            // K2 output [pair][n1][n2 / 2], columns 2c, 2c + 1 per element
     const float2* tw_hi;  // exp(-2 pi i 1024 t / N)
     const float2* tw_lo;  // exp(-2 pi i t / N), t < 1024
-    const float2* h;      // K4 input [n1][n2]
+    const float4* h;      // K4 input [n1][n2 / 2]: conj of the inverse row DFTs
     float* out;           // K4 output (n_v)
+    int out_vec;          // K4: out is 8-byte aligned
     float out_scale;
     // float-row variants (tangent and adjoint paths)
     const float* src;     // K2 input rows [node][row_stride] (float), or one row when single
     int single;           // K2: one real row (partner row zero), n_pairs = 1
-    int twiddle;          // K2: apply the four-step twiddle (row kernel without table)
     int ext;              // K2 float rows: 0, or the rows hold k in [-ext, n_v + ext) at offset k + ext
                           // (circular: k < 0 is FFT index n + k)
     int pair_base;        // K2: first output pair in y
@@ -240,22 +243,18 @@ struct ColFftArgs {       // K2 (forward column FFT) and K4 (inverse column FFT)
     double q_vmin, q_dv;  // v_k = q_vmin + k q_dv (cm-1)
 };
 
-struct VoigtArgs {        // K3 (row FFT + Voigt weights + pair reduction)
+struct VoigtArgs {        // K3 (row FFT + Voigt weights + pair reduction + inverse row DFT)
     FftLen f2;
-    int store_g;          // 1: one pair group: store the sums into G (no zeroing, no atomics)
-    int threads;          // block size (row_threads), >= n2 / 8
-    int pairs_per_pass;   // 2: two pairs as float4 elements; 1: one pair (long rows)
-    int row_twiddle_table;// 1: the row kernel applies the four-step twiddle from a
-                          // per-row shared table; 0: the column stage applies it
+    int units;            // pairs transformed side by side (row_shape)
+    int threads;          // block size (row_shape)
+    int bins;             // 1: store the summed bins (frequency form of g), no inverse
     int n1, n2;
     int64_t n;
     int n_pairs;
     int n_nodes;
     int NL;
-    const float2* y;
-    float2* g;            // accumulator [n1][n2]
-    const float2* tw_hi;  // exp(-2 pi i 1024 t / N)
-    const float2* tw_lo;  // exp(-2 pi i t / N), t < 1024
+    const float4* y;      // [pair][n1][n2 / 2]
+    float4* g;            // [n1][n2 / 2]
     float inv_ndv;        // 1 / (N dv)
     float half_fs;        // 1 / (2 dv)
     float alpha[kMaxAxis];    // (pi wG_l)^2 / (4 ln 2) * log2e
@@ -265,17 +264,6 @@ struct VoigtArgs {        // K3 (row FFT + Voigt weights + pair reduction)
     unsigned char nfold[kMaxNodes];
     int any_fold;
     int rowwise;          // 1: row r's transform uses alpha[r], beta[r] (skeleton rows, r < kMaxAxis)
-    int inv_fused;        // 1 (with store_g, one pair group): the CTA also applies the inverse
-                          // row DFT and inverse twiddle (K3b) to its row of sums before storing it
-};
-
-struct RowIfftArgs {      // K3b (inverse row FFT + twiddle, in place)
-    FftLen f2;
-    int n1, n2;
-    int64_t n;
-    float2* g;
-    const float2* tw_hi;
-    const float2* tw_lo;
 };
 
 // Gaussian stage of the merged layout: node rows of equal wL whose Gaussian
@@ -369,7 +357,7 @@ struct SlitArgs {
 
 struct AdjRowArgs {       // adjoint row stage: per pair, IFFT_row(Ghat (V_a + i V_b)) x twiddle
     VoigtArgs v;          // v.g holds Ghat [n1][n2] (FFT of the upstream gradient)
-    float2* y;            // output [pair][n1][n2]
+    float4* y;            // output [pair][n1][n2 / 2]
 };
 
 struct GradArgs {         // adjoint gather (reverse mode) and tangent scatter (forward mode)
@@ -431,7 +419,6 @@ int launch_scatter_auto(const ScatterArgs& a32, const ScatterArgs& a64, int grid
 int scatter_smem_optin(size_t* avail, bool wide);
 int launch_col_fft_fwd(const ColFftArgs& a, cudaStream_t st);
 int launch_row_fft_voigt(const VoigtArgs& a, cudaStream_t st);
-int launch_row_ifft(const RowIfftArgs& a, cudaStream_t st);
 int launch_col_ifft(const ColFftArgs& a, cudaStream_t st);
 // tangent / adjoint path (forward-mode and reverse-mode derivatives)
 int launch_col_fft_fwd_f(const ColFftArgs& a, cudaStream_t st);
@@ -454,14 +441,10 @@ int interp_decomp(const double* A, int S, int n, double tol, int r_max, int* sk,
                   double* err_out);
 int launch_slit_conv(const SlitArgs& a, int sms, cudaStream_t st);
 int launch_scatter_tangent(const GradArgs& a, int grid, cudaStream_t st);
-int col_block(int n1);               // columns per CTA of the column FFTs
-int row_threads(const FftLen& f);    // block size of the forward row kernel
-struct RowLayout {         // forward row kernel layout for rows of n2 points
-    int pairs;            // node pairs per element (2: float4, 1: float2)
-    int maxt;             // block size limit
-    int twr;              // per-row four-step twiddle table (else the column stage twiddles)
-    int stage;            // cp.async staging of the next two rows
+struct RowShape {
+    int units, threads;
 };
-RowLayout row_layout(int n2);
+// pairs side by side and threads of the row kernels (adjoint: k_row_ifft_adj)
+RowShape row_shape(const FftLen& f, int n1, int n_pairs, int sms, bool adjoint);
 
 }  // namespace rg

@@ -4,14 +4,7 @@
 //   k_scatter       fused per-line scaling + 2x2x2 scatter into a shared-memory
 //                   LDM tile, flushed once to HBM with plain stores
 //                   (replaces cmdFillLDM.comp:75-145 and the buffer clear)
-//   k_col_fft_fwd   first half of a four-step FFT: length-n1 DFTs down the
-//                   columns of two packed node rows + twiddle
-//   k_row_fft_voigt second half: length-n2 DFT of each row, times the analytic
-//                   Voigt FT of the node pair, summed over pairs
-//                   (replaces the R2C FFT + cmdApplyLineshapes.comp:51-90)
-//   k_row_ifft      inverse row DFTs + twiddle, in place
-//   k_col_ifft      inverse column DFTs, real part, scaled, first n_v samples
-//                   (replaces the C2R IFFT)
+//   k_col_fft_fwd, k_row_fft_voigt, k_col_ifft   the FFT stage (rg_fft.cu)
 // Two real node rows a, b are transformed as one complex row z = a + i b.
 // With W = V_a - i V_b, sum_j Z_j W_j = G and abscoeff = Re(IFFT(G)) / (N dv):
 // the Hermitian pairing of bins k and N-k is absorbed by taking the real part.
@@ -20,20 +13,14 @@
 #include <algorithm>
 #include <atomic>
 #include <cstdio>
-#include <type_traits>
 
-#include "rg_internal.h"
+#include "rg_device.cuh"
 
 namespace rg {
 
 // ---------------------------------------------------------------------------
 // small helpers
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ float ex2(float x) {
-    float y;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
 __device__ __forceinline__ float lg2(float x) {
     float y;
     asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
@@ -45,343 +32,6 @@ __device__ __forceinline__ void two_sum(float a, float b, float& s, float& e) {
     float bb = s - a;
     e = (a - (s - bb)) + (b - bb);
 }
-__device__ __forceinline__ float2 cmul(float2 a, float2 b) {
-    return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
-}
-__device__ __forceinline__ float2 cadd(float2 a, float2 b) { return make_float2(a.x + b.x, a.y + b.y); }
-__device__ __forceinline__ float2 csub(float2 a, float2 b) { return make_float2(a.x - b.x, a.y - b.y); }
-__device__ __forceinline__ float2 conjf2(float2 a) { return make_float2(a.x, -a.y); }
-// multiply by -i (forward-direction quarter turn)
-__device__ __forceinline__ float2 mul_mi(float2 a) { return make_float2(a.y, -a.x); }
-
-// ---------------------------------------------------------------------------
-// forward DFTs of radix 2, 3, 4, 5, 8 in registers (exp(-2 pi i n k / R))
-// ---------------------------------------------------------------------------
-__device__ __forceinline__ void dft2(float2* v) {
-    float2 a = v[0], b = v[1];
-    v[0] = cadd(a, b);
-    v[1] = csub(a, b);
-}
-__device__ __forceinline__ void dft4(float2* v) {
-    float2 s02 = cadd(v[0], v[2]), d02 = csub(v[0], v[2]);
-    float2 s13 = cadd(v[1], v[3]), d13 = mul_mi(csub(v[1], v[3]));
-    v[0] = cadd(s02, s13);
-    v[2] = csub(s02, s13);
-    v[1] = cadd(d02, d13);
-    v[3] = csub(d02, d13);
-}
-__device__ __forceinline__ void dft3(float2* v) {
-    const float c1 = -0.5f, s1 = 0.86602540378443864676f;   // cos/sin(2 pi / 3)
-    float2 t = cadd(v[1], v[2]);
-    float2 d = csub(v[1], v[2]);
-    float2 a0 = v[0];
-    v[0] = cadd(a0, t);
-    float2 m = make_float2(a0.x + c1 * t.x, a0.y + c1 * t.y);
-    // -i * s1 * d
-    float2 r = make_float2(s1 * d.y, -s1 * d.x);
-    v[1] = cadd(m, r);
-    v[2] = csub(m, r);
-}
-__device__ __forceinline__ void dft5(float2* v) {
-    const float c1 = 0.30901699437494742410f, s1 = 0.95105651629515357212f;  // 2 pi / 5
-    const float c2 = -0.80901699437494742410f, s2 = 0.58778525229247312917f; // 4 pi / 5
-    float2 a0 = v[0];
-    float2 t1 = cadd(v[1], v[4]), d1 = csub(v[1], v[4]);
-    float2 t2 = cadd(v[2], v[3]), d2 = csub(v[2], v[3]);
-    v[0] = make_float2(a0.x + t1.x + t2.x, a0.y + t1.y + t2.y);
-    float2 m1 = make_float2(a0.x + c1 * t1.x + c2 * t2.x, a0.y + c1 * t1.y + c2 * t2.y);
-    float2 m2 = make_float2(a0.x + c2 * t1.x + c1 * t2.x, a0.y + c2 * t1.y + c1 * t2.y);
-    // forward: X1 = m1 - i (s1 d1 + s2 d2), X4 = m1 + i (...)
-    float2 q1 = make_float2(s1 * d1.x + s2 * d2.x, s1 * d1.y + s2 * d2.y);
-    float2 q2 = make_float2(s2 * d1.x - s1 * d2.x, s2 * d1.y - s1 * d2.y);
-    v[1] = cadd(m1, mul_mi(q1));
-    v[4] = csub(m1, mul_mi(q1));
-    v[2] = cadd(m2, mul_mi(q2));
-    v[3] = csub(m2, mul_mi(q2));
-}
-__device__ __forceinline__ void dft8(float2* v) {
-    const float r = 0.70710678118654752440f;
-    // radix-2 split: even / odd halves
-    float2 e[4] = {v[0], v[2], v[4], v[6]};
-    float2 o[4] = {v[1], v[3], v[5], v[7]};
-    dft4(e);
-    dft4(o);
-    // twiddles w8^k = exp(-i pi k / 4), k = 0..3
-    float2 o1 = make_float2(r * (o[1].x + o[1].y), r * (o[1].y - o[1].x));
-    float2 o2 = mul_mi(o[2]);
-    float2 o3 = make_float2(r * (o[3].y - o[3].x), -r * (o[3].x + o[3].y));
-    v[0] = cadd(e[0], o[0]);
-    v[4] = csub(e[0], o[0]);
-    v[1] = cadd(e[1], o1);
-    v[5] = csub(e[1], o1);
-    v[2] = cadd(e[2], o2);
-    v[6] = csub(e[2], o2);
-    v[3] = cadd(e[3], o3);
-    v[7] = csub(e[3], o3);
-}
-
-// exp(-2 pi i M / N) at compile time: octant-free quadrant reduction of the
-// exact fraction M / N, then Taylor series on [0, pi/2) (double, ~1e-16)
-constexpr double kPiC = 3.14159265358979323846;
-__host__ __device__ constexpr double csin_q(double y) {
-    double t = y, s = y;
-    for (int k = 1; k < 14; ++k) {
-        t *= -y * y / ((2.0 * k) * (2.0 * k + 1.0));
-        s += t;
-    }
-    return s;
-}
-__host__ __device__ constexpr double ccos_q(double y) {
-    double t = 1.0, s = 1.0;
-    for (int k = 1; k < 14; ++k) {
-        t *= -y * y / ((2.0 * k - 1.0) * (2.0 * k));
-        s += t;
-    }
-    return s;
-}
-__host__ __device__ constexpr double ctw(int m, int n, bool sine) {
-    const int mm = ((m % n) + n) % n;
-    const int q = 4 * mm / n;                                  // quadrant
-    const double y = 2.0 * kPiC * (double)(4 * mm - q * n) / (4.0 * n);   // in [0, pi/2)
-    const double c = ccos_q(y), sn = csin_q(y);
-    if (!sine) return q == 0 ? c : q == 1 ? -sn : q == 2 ? -c : sn;
-    return q == 0 ? sn : q == 1 ? c : q == 2 ? -sn : -c;
-}
-template <int M, int N>
-struct TwConst {   // exp(-2 pi i M / N)
-    static constexpr float re = (float)ctw(M, N, false);
-    static constexpr float im = (float)-ctw(M, N, true);
-};
-template <int R>
-__device__ __forceinline__ void dftR(float2* v);
-
-// Stage 1 of a length-A B DFT, in place: for column n2 (N2), the A-point DFT
-// of v[B n1 + n2] over n1, each output k1 times exp(-2 pi i n2 k1 / (A B))
-// (compile-time constants), written back to v[B k1 + n2].
-template <int A, int B, int N2, int K1>
-__device__ __forceinline__ void twiddle_col(float2* v, const float2* t) {
-    if constexpr (K1 < A) {
-        constexpr int e = N2 * K1 % (A * B);
-        if constexpr (e == 0)
-            v[B * K1 + N2] = t[K1];
-        else
-            v[B * K1 + N2] = cmul(t[K1], make_float2(TwConst<e, A * B>::re, TwConst<e, A * B>::im));
-        twiddle_col<A, B, N2, K1 + 1>(v, t);
-    }
-}
-template <int A, int B, int N2>
-__device__ __forceinline__ void dft_stage1(float2* v) {
-    if constexpr (N2 < B) {
-        float2 t[A];
-#pragma unroll
-        for (int n1 = 0; n1 < A; ++n1) t[n1] = v[B * n1 + N2];
-        dftR<A>(t);
-        twiddle_col<A, B, N2, 0>(v, t);
-        dft_stage1<A, B, N2 + 1>(v);
-    }
-}
-
-// DFT of length A B in registers, natural order in and out (Cooley-Tukey,
-// n = B n1 + n2, k = k1 + A k2), in place: stage 1 above, then the B-point
-// DFTs of v[B k1 + n2] over n2 back into the same slots, which leaves
-// X[k1 + A k2] in v[B k1 + k2]; a compile-time register permutation restores
-// natural order.
-template <int A, int B>
-__device__ __forceinline__ void dftAB(float2* v) {
-    constexpr int N = A * B;
-    dft_stage1<A, B, 0>(v);
-#pragma unroll
-    for (int k1 = 0; k1 < A; ++k1) dftR<B>(v + B * k1);
-    float2 t[N];
-#pragma unroll
-    for (int r = 0; r < N; ++r) t[r] = v[B * (r % A) + r / A];
-#pragma unroll
-    for (int r = 0; r < N; ++r) v[r] = t[r];
-}
-
-// radices of the FFT plans: 2, 3, 4, 5, 8 and the composites 6, 9, 10, 12 of
-// the small factors
-template <int R>
-__device__ __forceinline__ void dftR(float2* v) {
-    if constexpr (R == 2) dft2(v);
-    else if constexpr (R == 3) dft3(v);
-    else if constexpr (R == 4) dft4(v);
-    else if constexpr (R == 5) dft5(v);
-    else if constexpr (R == 8) dft8(v);
-    else if constexpr (R == 6) dftAB<2, 3>(v);
-    else if constexpr (R == 9) dftAB<3, 3>(v);
-    else if constexpr (R == 10) dftAB<2, 5>(v);
-    else if constexpr (R == 12) dftAB<4, 3>(v);
-}
-// dispatch of a run-time radix to f(integral_constant<R>), instantiating only
-// the radices up to MAXR (other radices never reach the call)
-template <int MAXR = 12, class F>
-__device__ __forceinline__ void with_radix(int R, F&& f) {
-    switch (R) {
-        case 2: f(std::integral_constant<int, 2>()); break;
-        case 3: f(std::integral_constant<int, 3>()); break;
-        case 4: f(std::integral_constant<int, 4>()); break;
-        case 5: f(std::integral_constant<int, 5>()); break;
-        case 6: f(std::integral_constant<int, 6>()); break;
-        case 9: if constexpr (MAXR >= 9) f(std::integral_constant<int, 9>()); break;
-        case 10: if constexpr (MAXR >= 10) f(std::integral_constant<int, 10>()); break;
-        case 12: if constexpr (MAXR >= 12) f(std::integral_constant<int, 12>()); break;
-        default: f(std::integral_constant<int, 8>()); break;
-    }
-}
-
-// Multiply v[1..R-1] by w^r, w = tw[s] (tw[t] = exp(-2 pi i t / L)); three
-// table reads at most, the other powers by complex products.
-template <int R>
-__device__ __forceinline__ void twiddle(float2* v, const float2* __restrict__ tw, int s) {
-    const float2 w1 = __ldg(&tw[s]);
-    if (R == 2) {
-        v[1] = cmul(v[1], w1);
-    } else if (R == 3) {
-        v[1] = cmul(v[1], w1);
-        v[2] = cmul(v[2], __ldg(&tw[2 * s]));
-    } else if (R == 4) {
-        const float2 w2 = __ldg(&tw[2 * s]);
-        v[1] = cmul(v[1], w1);
-        v[2] = cmul(v[2], w2);
-        v[3] = cmul(v[3], cmul(w1, w2));
-    } else if (R == 5) {
-        const float2 w2 = __ldg(&tw[2 * s]);
-        v[1] = cmul(v[1], w1);
-        v[2] = cmul(v[2], w2);
-        v[3] = cmul(v[3], cmul(w1, w2));
-        v[4] = cmul(v[4], cmul(w2, w2));
-    } else if (R == 8) {
-        const float2 w2 = __ldg(&tw[2 * s]);
-        const float2 w4 = __ldg(&tw[4 * s]);
-        const float2 w3 = cmul(w1, w2);
-        v[1] = cmul(v[1], w1);
-        v[2] = cmul(v[2], w2);
-        v[3] = cmul(v[3], w3);
-        v[4] = cmul(v[4], w4);
-        v[5] = cmul(v[5], cmul(w1, w4));
-        v[6] = cmul(v[6], cmul(w2, w4));
-        v[7] = cmul(v[7], cmul(w3, w4));
-    } else {   // composite radix: w^r by products, from the table at every 4th power
-        float2 w = w1;
-#pragma unroll
-        for (int r = 1; r < R; ++r) {
-            if (r > 1) w = (r % 4 == 0) ? __ldg(&tw[r * s]) : cmul(w, w1);
-            v[r] = cmul(v[r], w);
-        }
-    }
-}
-
-// One Stockham autosort pass over a single transform of length L held in
-// shared memory (sub-transforms of length Ns before the pass): butterfly j
-// reads in[j + r L/R], twiddles by w_{Ns R}^{r (j mod Ns)} and writes
-// out[(j / Ns) Ns R + (j mod Ns) + r Ns].
-// Row buffers are padded by one element every 16 (index i lives at
-// rp(i) = i + i/16) so that the stride-R writes of the first pass spread over
-// the banks.
-__device__ __forceinline__ int rp(int i) { return i + (i >> 4); }
-__host__ __device__ constexpr int row_buf_len(int n) { return n + (n >> 4) + 1; }
-
-template <int R, bool PIN, bool POUT>
-__device__ __forceinline__ void row_pass(const float2* __restrict__ in, float2* __restrict__ out, int L,
-                                         int Ns, unsigned mag, const float2* __restrict__ tw) {
-    const int M = L / R;
-    const int twstep = L / (Ns * R);
-    for (int j = threadIdx.x; j < M; j += blockDim.x) {
-        const int q = Ns == 1 ? j : (int)__umulhi((unsigned)j, mag);
-        const int k = j - q * Ns;
-        float2 v[R];
-#pragma unroll
-        for (int r = 0; r < R; ++r) v[r] = in[PIN ? rp(j + r * M) : j + r * M];
-        if (Ns > 1) twiddle<R>(v, tw, k * twstep);
-        dftR<R>(v);
-        const int base = q * Ns * R + k;
-#pragma unroll
-        for (int r = 0; r < R; ++r) out[POUT ? rp(base + r * Ns) : base + r * Ns] = v[r];
-    }
-}
-
-template <bool PIN, bool POUT>
-__device__ __forceinline__ void row_pass_r(int R, const float2* in, float2* out, int L, int Ns, unsigned mag,
-                                           const float2* tw) {
-    with_radix(R, [&](auto rc) { row_pass<decltype(rc)::value, PIN, POUT>(in, out, L, Ns, mag, tw); });
-}
-
-// Forward DFT of one row in shared memory; buf0 holds the input (plain
-// layout).  Only the first pass's strided writes (and the second pass's reads
-// of them) use the padded layout rp(); later passes access in plain layout.
-// Returns the buffer holding the result; *padded tells its layout.  Ends with
-// __syncthreads().
-__device__ float2* fft_row(float2* buf0, float2* buf1, const FftLen& P, bool* padded) {
-    float2* in = buf0;
-    float2* out = buf1;
-    for (int p = 0; p < P.npass; ++p) {
-        const int R = P.radix[p];
-        const int Ns = P.ns[p];
-        const unsigned mag = P.mag[p];
-        if (p == 0)
-            row_pass_r<false, true>(R, in, out, P.L, Ns, mag, P.tw);
-        else if (p == 1)
-            row_pass_r<true, false>(R, in, out, P.L, Ns, mag, P.tw);
-        else
-            row_pass_r<false, false>(R, in, out, P.L, Ns, mag, P.tw);
-        __syncthreads();
-        float2* t = in;
-        in = out;
-        out = t;
-    }
-    *padded = P.npass == 1;
-    return in;
-}
-
-// Column FFT of length N1 in {8, 64, 512} = 8^d, B columns per CTA, N1/8
-// threads per column, one radix-8 butterfly per thread and pass with the
-// eight values in registers; passes exchange through one shared buffer
-// [N1][B].  On entry v[q] = x[j + q N1/8] of column b; on return
-// v[r] = X[j + r N1/8].
-template <int N1>
-struct ColShape {
-    static constexpr int TPC = N1 / 8;
-    static constexpr int B = N1 == 512 ? 8 : 32;
-    static constexpr int THREADS = TPC * B;
-};
-
-template <int N1>
-__device__ __forceinline__ void col_fft8(float2 (&v)[8], float2* sm, int j, int b,
-                                         const float2* __restrict__ tw1) {
-    constexpr int TPC = ColShape<N1>::TPC;
-    constexpr int B = ColShape<N1>::B;
-    dft8(v);
-    if constexpr (N1 > 8) {
-        // pass 1 (Ns = 1) writes out[8 j + r]
-#pragma unroll
-        for (int r = 0; r < 8; ++r) sm[(8 * j + r) * B + b] = v[r];
-        __syncthreads();
-#pragma unroll
-        for (int r = 0; r < 8; ++r) v[r] = sm[(j + r * TPC) * B + b];
-        const int k = j & 7;
-        twiddle<8>(v, tw1, (N1 / 64) * k);      // w_64^{r k}
-        dft8(v);
-        if constexpr (N1 > 64) {
-            __syncthreads();
-            // pass 2 (Ns = 8) writes out[(j - k) 8 + k + 8 r]
-#pragma unroll
-            for (int r = 0; r < 8; ++r) sm[((j - k) * 8 + k + 8 * r) * B + b] = v[r];
-            __syncthreads();
-#pragma unroll
-            for (int r = 0; r < 8; ++r) v[r] = sm[(j + r * TPC) * B + b];
-            twiddle<8>(v, tw1, j);              // w_512^{r j}
-            dft8(v);
-        }
-    }
-}
-
-// exp(-2 pi i t / N) from a two-level table (t = hi * 1024 + lo)
-__device__ __forceinline__ float2 twiddle_n(const float2* __restrict__ hi, const float2* __restrict__ lo,
-                                            int t) {
-    return cmul(__ldg(&hi[t >> 10]), __ldg(&lo[t & 1023]));
-}
-
 // ---------------------------------------------------------------------------
 // line preparation at upload: (hi, lo) split of v0 and log2 of the intensity
 // ---------------------------------------------------------------------------
@@ -1064,517 +714,6 @@ __global__ void __launch_bounds__(kScatThreads, 1) k_scatter_auto(const ScatterA
 }
 
 // ---------------------------------------------------------------------------
-// K2: forward column FFT (length n1) of packed node pairs
-// ---------------------------------------------------------------------------
-// Column-stage output X[k1] of column n2i into y[pair][k1][n2i], times the
-// four-step twiddle w_N^{n2i k1} when the row stage does not apply it
-// (a.twiddle): w for k1 = j + r N1/8 is w_N^{n2i j} (w_N^{n2i N1/8})^r, two
-// table reads and a product recurrence (rounding grows to ~8 ulp at r = 7).
-template <int N1>
-__device__ __forceinline__ void store_twiddled(float2 (&v)[8], const ColFftArgs& a, int pair, int j, int n2i) {
-    constexpr int TPC = ColShape<N1>::TPC;
-    float2* y = a.y + (int64_t)(a.pair_base + pair) * N1 * a.n2;
-    if (a.twiddle) {
-        float2 w = twiddle_n(a.tw_hi, a.tw_lo, n2i * j);
-        const float2 step = twiddle_n(a.tw_hi, a.tw_lo, n2i * TPC);
-#pragma unroll
-        for (int r = 0; r < 8; ++r) {
-            v[r] = cmul(v[r], w);
-            w = cmul(w, step);
-        }
-    }
-#pragma unroll
-    for (int r = 0; r < 8; ++r) y[(int64_t)(j + r * TPC) * a.n2 + n2i] = v[r];
-}
-
-template <int N1>
-__global__ void __launch_bounds__(ColShape<N1>::THREADS, 3) k_col_fft_fwd(const ColFftArgs a) {
-    constexpr int TPC = ColShape<N1>::TPC;
-    constexpr int B = ColShape<N1>::B;
-    extern __shared__ float2 sm[];
-    const int b = threadIdx.x % B;
-    const int j = threadIdx.x / B;
-    const int c0 = blockIdx.x * B;
-    const int pair = blockIdx.y;
-    auto node_of = [&](int v) {   // -1: zero row (padding of an odd n_L block)
-        if (!a.map_n) return v;
-        const int m = v % a.map_NLv;
-        return m < a.map_NL ? a.map_l[v / a.map_NLv] * a.map_NL + m : -1;
-    };
-    const int na = node_of(2 * pair), nb = node_of(2 * pair + 1);
-    const float* ra = na >= 0 ? a.ldm + (int64_t)na * a.row_stride : nullptr;
-    const float* rb = nb >= 0 ? a.ldm + (int64_t)nb * a.row_stride : nullptr;
-    const int n2i = c0 + b;
-    float2 v[8];
-#pragma unroll
-    for (int q = 0; q < 8; ++q) {
-        const int64_t nidx = (int64_t)(j + q * TPC) * a.n2 + n2i;
-        v[q] = nidx < a.n_v ? make_float2(ra ? __ldg(&ra[nidx]) : 0.f, rb ? __ldg(&rb[nidx]) : 0.f)
-                            : make_float2(0.f, 0.f);
-    }
-    col_fft8<N1>(v, sm, j, b, a.f1.tw);
-    store_twiddled<N1>(v, a, pair, j, n2i);
-}
-
-// ---------------------------------------------------------------------------
-// K3: row FFT (length n2) of each pair, Voigt-FT weights, sum over pairs
-// ---------------------------------------------------------------------------
-constexpr int kRowThreads = 256;      // inverse row kernel
-
-struct NodeV {
-    float al, bm, nrm;
-    int nf;
-};
-
-__device__ __forceinline__ NodeV node_params(const VoigtArgs& a, int node) {
-    const int l = a.rowwise ? node : node / a.NL;
-    const int m = a.rowwise ? node : node - l * a.NL;
-    NodeV n;
-    n.al = a.alpha[l];
-    n.bm = a.beta[m];
-    n.nrm = a.norm[node];
-    n.nf = a.any_fold ? (int)a.nfold[node] : 0;
-    return n;
-}
-
-// folded copies of the Voigt FT (broadening.py:1914-1926): alias frequencies
-// q/(2 dv) + (f or 1/(2 dv) - f); rare, kept out of line
-__device__ __noinline__ float voigt_folds(float al, float bm, int nf, float f, float half_fs) {
-    float v = 0.f;
-    for (int q = 1; q <= nf; ++q) {
-        const float fq = q * half_fs + ((q & 1) ? half_fs - f : f);
-        v += ex2(-fmaf(al * fq, fq, bm * fq));
-    }
-    return v;
-}
-
-__device__ __forceinline__ float voigt_eval(const NodeV& n, float f, float half_fs) {
-    float v = ex2(-fmaf(n.al * f, f, n.bm * f));
-    if (n.nf) v += voigt_folds(n.al, n.bm, n.nf, f, half_fs);
-    return v * n.nrm;
-}
-
-// Unfolded Voigt FT with the normalisation folded into the exponent:
-// nrm 2^-(al f^2 + bm f) = 2^(lnrm - bm f - al f^2), two FMAs and one ex2.
-struct NodeF {
-    float nal, nbm, lnrm;
-};
-__device__ __forceinline__ NodeF node_fast(const VoigtArgs& a, int node) {
-    const int l = a.rowwise ? node : node / a.NL;
-    NodeF n;
-    n.nal = -a.alpha[l];
-    n.nbm = -a.beta[a.rowwise ? node : node - l * a.NL];
-    n.lnrm = a.lnorm[node];
-    return n;
-}
-__device__ __forceinline__ float voigt_fast(const NodeF& n, float f, float f2) {
-    return ex2(fmaf(n.nal, f2, fmaf(n.nbm, f, n.lnrm)));
-}
-
-// PAIRS = 2: two pairs travel together through the row transform as float4
-// elements (row A in .xy, row B in .zw), sharing index arithmetic, twiddle
-// loads and shared-memory instructions; buffers use rp8(i) = i + i/8, which
-// keeps every 16-byte access pattern of the passes conflict-free.
-// PAIRS = 1 (long rows): float2 elements, rp16(i) = i + i/16.
-__device__ __forceinline__ int rp8(int i) { return i + (i >> 3); }
-__device__ __forceinline__ int rp16(int i) { return i + (i >> 4); }
-template <int PAIRS> struct RowT;
-template <> struct RowT<2> {
-    using E = float4;
-    __device__ static int pad(int i) { return rp8(i); }
-    __host__ __device__ static constexpr int len(int n) { return n + (n >> 3) + 1; }
-    __device__ static void split(E t, float2& a, float2& b) {
-        a = make_float2(t.x, t.y);
-        b = make_float2(t.z, t.w);
-    }
-    __device__ static E join(float2 a, float2 b) { return make_float4(a.x, a.y, b.x, b.y); }
-};
-template <> struct RowT<1> {
-    using E = float2;
-    __device__ static int pad(int i) { return rp16(i); }
-    // even, so the second work buffer starts 16-byte aligned (cp.async staging)
-    __host__ __device__ static constexpr int len(int n) { return n + (n >> 4) + 2; }
-    __device__ static void split(E t, float2& a, float2& b) {
-        a = t;
-        b = make_float2(0.f, 0.f);
-    }
-    __device__ static E join(float2 a, float2) { return a; }
-};
-
-// Row-pass twiddle sources, tw(t) = exp(-2 pi i t / n2): the global table,
-// or a two-level table in shared memory, hi[t / 32] lo[t % 32] (one more
-// rounding; used by the long-row layouts, whose n2-point table would not stay
-// in the L1 left beside their work buffers).
-struct TwGlobal {
-    const float2* __restrict__ tw;
-    __device__ __forceinline__ float2 operator()(int t) const { return __ldg(&tw[t]); }
-};
-struct TwShared {
-    const float2* hi;
-    const float2* lo;
-    __device__ __forceinline__ float2 operator()(int t) const { return cmul(hi[t >> 5], lo[t & 31]); }
-};
-
-template <int R, int PAIRS, class TW>
-__device__ __forceinline__ void twiddleP(float2* A, float2* B, const TW& tw, int s) {
-    if constexpr (R == 2 || R == 3 || R == 4 || R == 5 || R == 8) {
-        float2 w[R];
-        w[0] = make_float2(1.f, 0.f);
-        w[1] = tw(s);
-        if (R >= 3) w[2] = tw(2 * s);
-        if (R >= 4) w[3] = cmul(w[1], w[2]);
-        if (R == 5) w[4] = cmul(w[2], w[2]);
-        if (R == 8) {
-            w[4] = tw(4 * s);
-            w[5] = cmul(w[1], w[4]);
-            w[6] = cmul(w[2], w[4]);
-            w[7] = cmul(w[3], w[4]);
-        }
-#pragma unroll
-        for (int r = 1; r < R; ++r) {
-            A[r] = cmul(A[r], w[r]);
-            if (PAIRS == 2) B[r] = cmul(B[r], w[r]);
-        }
-    } else {   // composite radix: w^r by products, from the table at every 4th power
-        const float2 w1 = tw(s);
-        float2 w = w1;
-#pragma unroll
-        for (int r = 1; r < R; ++r) {
-            if (r > 1) w = (r % 4 == 0) ? tw(r * s) : cmul(w, w1);
-            A[r] = cmul(A[r], w);
-            if (PAIRS == 2) B[r] = cmul(B[r], w);
-        }
-    }
-}
-
-template <int R, int PAIRS, class TW>
-__device__ __forceinline__ void row_mid(const typename RowT<PAIRS>::E* __restrict__ in,
-                                        typename RowT<PAIRS>::E* __restrict__ out, int L, int Ns, unsigned mag,
-                                        const TW& tw) {
-    const int M = L / R;
-    const int twstep = L / (Ns * R);
-    for (int j = threadIdx.x; j < M; j += blockDim.x) {
-        const int q = Ns == 1 ? j : (int)__umulhi((unsigned)j, mag);
-        const int k = j - q * Ns;
-        float2 A[R], B[R];
-#pragma unroll
-        for (int r = 0; r < R; ++r) RowT<PAIRS>::split(in[RowT<PAIRS>::pad(j + r * M)], A[r], B[r]);
-        if (Ns > 1) twiddleP<R, PAIRS, TW>(A, B, tw, k * twstep);
-        dftR<R>(A);
-        if (PAIRS == 2) dftR<R>(B);
-        const int base = q * Ns * R + k;
-#pragma unroll
-        for (int r = 0; r < R; ++r) out[RowT<PAIRS>::pad(base + r * Ns)] = RowT<PAIRS>::join(A[r], B[r]);
-    }
-}
-
-// two work buffers, the optional twiddle table, and the optional staging
-// buffer of the next two rows
-template <int PAIRS>
-__host__ __device__ inline size_t row_voigt_smem(int n2, bool with_twr, bool with_stage, bool with_tws = false) {
-    return 2 * (size_t)RowT<PAIRS>::len(n2) * sizeof(typename RowT<PAIRS>::E) +
-           (with_twr ? (size_t)n2 * sizeof(float2) : 0) + (with_stage ? 2 * (size_t)n2 * sizeof(float2) : 0) +
-           (with_tws ? (size_t)(n2 / 32 + 32) * sizeof(float2) : 0);
-}
-
-// Layouts of the forward row kernel: MAXT threads at most, and the block is
-// at least the n2/8 butterflies of the last (radix-8) pass, so each thread
-// owns one butterfly's 8 output bins and their accumulators.
-constexpr int kRowMaxT2 = 384;    // PAIRS = 2, two CTAs per SM (n2 <= 3072)
-constexpr int kRowMaxT2L = 768;   // PAIRS = 2, one CTA per SM (n2 <= 6144, work buffers only)
-constexpr int kRowMaxT1 = 1024;   // PAIRS = 1, long rows (n2 <= 8192)
-
-// cp.async staging of the next rows of a pair group (16-byte copies that
-// bypass L1, completed with wait_group before the first pass reads them)
-__device__ __forceinline__ void stage_rows(float2* dst, const float2* ya, const float2* yb, int n2) {
-    const int chunks = n2 / 2;   // 16-byte chunks per row
-    for (int c = threadIdx.x; c < 2 * chunks; c += blockDim.x) {
-        const bool second = c >= chunks;
-        const float2* src = (second ? yb : ya) + 2 * (c - (second ? chunks : 0));
-        if (second && !yb) continue;
-        const uint32_t d = smem_u32(dst + 2 * c);
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
-    }
-    asm volatile("cp.async.commit_group;" ::: "memory");
-}
-__device__ __forceinline__ void stage_wait() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
-
-// first pass from the staged rows (stage = [row a | row b], n2 each; row a
-// only for PAIRS = 1)
-// first pass (sub-transform length 1) from the staged rows: (x four-step
-// twiddle from the per-row table twr, when TWR; otherwise the column stage
-// applied it) -> registers -> smem
-template <int R, int PAIRS, bool TWR>
-__device__ __forceinline__ void row_first_staged(const float2* stage, bool two, const float2* twr,
-                                                 typename RowT<PAIRS>::E* out, int L) {
-    const int M = L / R;
-    for (int j = threadIdx.x; j < M; j += blockDim.x) {
-        float2 A[R], B[R];
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-            A[r] = stage[j + r * M];
-            B[r] = PAIRS == 2 && two ? stage[L + j + r * M] : make_float2(0.f, 0.f);
-            if (TWR) {
-                const float2 w = twr[j + r * M];
-                A[r] = cmul(A[r], w);
-                B[r] = cmul(B[r], w);
-            }
-        }
-        dftR<R>(A);
-        if (PAIRS == 2) dftR<R>(B);
-#pragma unroll
-        for (int r = 0; r < R; ++r) out[RowT<PAIRS>::pad(j * R + r)] = RowT<PAIRS>::join(A[r], B[r]);
-    }
-}
-
-// STAGE: the next two rows are staged in a buffer of their own.  SF: the next
-// rows are staged in the work buffer that the last pass does not read, and
-// the first pass reads them from there (the buffers swap roles).
-template <int PAIRS, int MAXT, bool TWR, bool STAGE, bool TWS, bool SF>
-__global__ void __launch_bounds__(MAXT, MAXT <= 384 ? 2 : 1) k_row_fft_voigt(const VoigtArgs a) {
-    static_assert(STAGE || SF, "the forward row kernel stages its rows");
-    using E = typename RowT<PAIRS>::E;
-    extern __shared__ float4 sm4[];
-    const int n2 = a.n2;
-    const int len = RowT<PAIRS>::len(n2);
-    E* buf0 = reinterpret_cast<E*>(sm4);
-    E* buf1 = buf0 + len;
-    float2* twr = TWR ? reinterpret_cast<float2*>(buf1 + len) : nullptr;
-    // STAGE (two pairs): the next two rows are staged with cp.async during the passes
-    float2* stage = STAGE ? reinterpret_cast<float2*>(buf1 + len) + (TWR ? n2 : 0) : nullptr;
-    const int k1 = blockIdx.x;
-    const FftLen& P = a.f2;
-    // TWS: two-level pass twiddle table after the other buffers (made visible
-    // by the barrier after the first pass)
-    float2* tws = TWS ? reinterpret_cast<float2*>(buf1 + len) + (TWR ? n2 : 0) + (STAGE ? 2 * n2 : 0) : nullptr;
-    if (TWS) {
-        for (int t = threadIdx.x; t < n2 / 32; t += blockDim.x) tws[t] = __ldg(&P.tw[32 * t]);
-        for (int t = threadIdx.x; t < 32; t += blockDim.x) tws[n2 / 32 + t] = __ldg(&P.tw[t]);
-    }
-    using TwT = typename std::conditional<TWS, TwShared, TwGlobal>::type;
-    TwT twp;
-    if constexpr (TWS) twp = TwShared{tws, tws + n2 / 32};
-    else twp = TwGlobal{P.tw};
-    if (TWR)
-        for (int t = threadIdx.x; t < n2; t += blockDim.x) twr[t] = twiddle_n(a.tw_hi, a.tw_lo, k1 * t);
-    const int n = (int)a.n;
-    const int j0 = blockIdx.y * kPairGroup;
-    const int j1 = min(j0 + kPairGroup, a.n_pairs);
-    const int ML = n2 / 8;    // butterflies of the last pass (radix 8, sub-length ML)
-    const int jl = threadIdx.x;
-    float2 acc[8];
-#pragma unroll
-    for (int r = 0; r < 8; ++r) acc[r] = make_float2(0.f, 0.f);
-
-    auto row_ptr = [&](int jj) { return a.y + ((int64_t)jj * a.n1 + k1) * n2; };
-    auto stage_group = [&](float2* dst, int jj) {   // rows of pair group jj (two for PAIRS = 2)
-        stage_rows(dst, row_ptr(jj), PAIRS == 2 && jj + 1 < j1 ? row_ptr(jj + 1) : nullptr, n2);
-    };
-    E* wbuf = buf0;   // first-pass output
-    E* fbuf = buf1;   // SF: the staged rows of the current pair group
-    if (STAGE && j0 < j1) stage_group(stage, j0);
-    if (SF && j0 < j1) stage_group(reinterpret_cast<float2*>(fbuf), j0);
-    for (int j = j0; j < j1; j += PAIRS) {
-        const bool two = PAIRS == 2 && j + 1 < j1;
-        if (STAGE || SF) {
-            const float2* src = STAGE ? stage : reinterpret_cast<const float2*>(fbuf);
-            stage_wait();
-            __syncthreads();   // staged rows (and the twiddle tables) visible to all threads
-            with_radix(P.radix[0], [&](auto rc) {
-                row_first_staged<decltype(rc)::value, PAIRS, TWR>(src, two, twr, wbuf, n2);
-            });
-            __syncthreads();   // stage consumed: prefetch the next two rows under the remaining passes
-            if (STAGE && j + 2 < j1) stage_group(stage, j + 2);
-        }
-        E* in = wbuf;
-        E* out = fbuf;
-        for (int p = 1; p < P.npass - 1; ++p) {
-            const int Ns = P.ns[p];
-            const unsigned mag = P.mag[p];
-            with_radix<kMidRadixMax>(P.radix[p], [&](auto rc) {
-                row_mid<decltype(rc)::value, PAIRS, TwT>(in, out, n2, Ns, mag, twp);
-            });
-            __syncthreads();
-            E* t = in;
-            in = out;
-            out = t;
-        }
-        // `out` is free until the next first pass: stage the next pair group there
-        if (SF && j + PAIRS < j1) stage_group(reinterpret_cast<float2*>(out), j + PAIRS);
-        // last pass (radix 8, sub-length ML, no shuffle: output t = jl + r ML),
-        // Voigt weights and accumulation in registers
-        if (jl < ML) {
-            float2 A[8], B[8];
-#pragma unroll
-            for (int r = 0; r < 8; ++r) RowT<PAIRS>::split(in[RowT<PAIRS>::pad(jl + r * ML)], A[r], B[r]);
-            twiddleP<8, PAIRS, TwT>(A, B, twp, jl);   // w_{n2}^{r jl}
-            dft8(A);
-            if (PAIRS == 2) dft8(B);
-            if (!a.any_fold) {
-                const NodeF A0 = node_fast(a, 2 * j), A1 = node_fast(a, 2 * j + 1);
-                NodeF B0 = A0, B1 = A1;
-                if (two) {
-                    B0 = node_fast(a, 2 * j + 2);
-                    B1 = node_fast(a, 2 * j + 3);
-                }
-#pragma unroll
-                for (int r = 0; r < 8; ++r) {
-                    const int kk = k1 + a.n1 * (jl + r * ML);
-                    const float f = (float)min(kk, n - kk) * a.inv_ndv;
-                    const float f2 = f * f;
-                    const float va = voigt_fast(A0, f, f2), vb = voigt_fast(A1, f, f2);
-                    float2 c = acc[r];
-                    c.x += A[r].x * va + A[r].y * vb;
-                    c.y += A[r].y * va - A[r].x * vb;
-                    if (two) {
-                        const float wa = voigt_fast(B0, f, f2), wb = voigt_fast(B1, f, f2);
-                        c.x += B[r].x * wa + B[r].y * wb;
-                        c.y += B[r].y * wa - B[r].x * wb;
-                    }
-                    acc[r] = c;
-                }
-            } else {
-                const NodeV A0 = node_params(a, 2 * j), A1 = node_params(a, 2 * j + 1);
-#pragma unroll
-                for (int r = 0; r < 8; ++r) {
-                    const int kk = k1 + a.n1 * (jl + r * ML);
-                    const float f = (float)min(kk, n - kk) * a.inv_ndv;
-                    const float va = voigt_eval(A0, f, a.half_fs);
-                    const float vb = voigt_eval(A1, f, a.half_fs);
-                    float2 c = acc[r];
-                    c.x += A[r].x * va + A[r].y * vb;
-                    c.y += A[r].y * va - A[r].x * vb;
-                    acc[r] = c;
-                }
-                if (two) {
-                    const NodeV B0 = node_params(a, 2 * j + 2), B1 = node_params(a, 2 * j + 3);
-#pragma unroll
-                    for (int r = 0; r < 8; ++r) {
-                        const int kk = k1 + a.n1 * (jl + r * ML);
-                        const float f = (float)min(kk, n - kk) * a.inv_ndv;
-                        const float wa = voigt_eval(B0, f, a.half_fs);
-                        const float wb = voigt_eval(B1, f, a.half_fs);
-                        float2 c = acc[r];
-                        c.x += B[r].x * wa + B[r].y * wb;
-                        c.y += B[r].y * wa - B[r].x * wb;
-                        acc[r] = c;
-                    }
-                }
-            }
-        }
-        __syncthreads();
-        if (SF) {   // the staged rows are in `out`; the next first pass writes `in`
-            wbuf = in;
-            fbuf = out;
-        }
-    }
-    if (a.inv_fused) {
-        // K3b on the CTA's own sums: inverse DFT = conj(forward DFT(conj(G))),
-        // through the work buffers (free after the last pair group), then the
-        // inverse four-step twiddle w_N^{-t k1}; the row is stored once
-        float2* f0 = reinterpret_cast<float2*>(sm4);
-        float2* f1 = f0 + row_buf_len(n2);
-        if (jl < ML) {
-#pragma unroll
-            for (int r = 0; r < 8; ++r) f0[jl + r * ML] = conjf2(acc[r]);
-        }
-        __syncthreads();
-        bool padded;
-        const float2* res = fft_row(f0, f1, a.f2, &padded);
-        float2* g = a.g + (int64_t)k1 * n2;
-        for (int t = threadIdx.x; t < n2; t += blockDim.x) {
-            float2 z = conjf2(res[padded ? rp(t) : t]);
-            if (k1 && t) z = cmul(z, conjf2(twiddle_n(a.tw_hi, a.tw_lo, t * k1)));
-            g[t] = z;
-        }
-        return;
-    }
-    if (jl < ML) {
-        float2* g = a.g + (int64_t)k1 * n2;
-        if (a.store_g && gridDim.y == 1) {   // the only pair group of this row: plain stores
-#pragma unroll
-            for (int r = 0; r < 8; ++r) g[jl + r * ML] = acc[r];
-        } else {
-#pragma unroll
-            for (int r = 0; r < 8; ++r) atomicAdd(&g[jl + r * ML], acc[r]);
-        }
-    }
-}
-
-// ---------------------------------------------------------------------------
-// K3b: inverse row FFT (length n2) and inverse twiddle w_N^{-n2 k1}, in place
-// ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(kRowThreads) k_row_ifft(const RowIfftArgs a) {
-    extern __shared__ float2 sm[];
-    const int n2 = a.n2;
-    float2* buf0 = sm;
-    float2* buf1 = sm + row_buf_len(n2);
-    const int k1 = blockIdx.x;
-    float2* g = a.g + (int64_t)k1 * n2;
-    for (int t = threadIdx.x; t < n2; t += blockDim.x) buf0[t] = conjf2(g[t]);
-    __syncthreads();
-    // inverse DFT = conj(forward DFT(conj(x)))
-    bool padded;
-    const float2* res = fft_row(buf0, buf1, a.f2, &padded);
-    for (int t = threadIdx.x; t < n2; t += blockDim.x) {
-        float2 z = conjf2(res[padded ? rp(t) : t]);
-        if (k1 && t) z = cmul(z, conjf2(twiddle_n(a.tw_hi, a.tw_lo, t * k1)));
-        g[t] = z;
-    }
-}
-
-// ---------------------------------------------------------------------------
-// K4: inverse column FFT (length n1), real part, scaled, first n_v samples
-// ---------------------------------------------------------------------------
-// Post-processing epilogue (radis/lbl/factory.py:1284-1297 and
-// radis/spectrum/equations.py:21-44): absorbance A L, emissivity
-// -expm1(-A L), transmittance 1 - emissivity, radiance emissivity x Planck
-// (radis/phys/blackbody.py:35-74, mW / cm2 / sr / nm at lambda = 1e7/nu nm).
-__device__ __forceinline__ void quantities_at(const ColFftArgs& a, int64_t k, float A) {
-    const float tau = A * a.q_scale * a.q_path;      // absorbance in physical units
-    const float eps = -expm1f(-tau);
-    const float nu = (float)(a.q_vmin + a.q_dv * (double)k);
-    const float lam = 0.01f / nu;                    // m
-    // 2 h c^2 / lambda^5 / expm1(h c / (lambda k T)) W m-3 sr-1 -> mW cm-2 sr-1 nm-1 (x 1e-10)
-    const float l2 = lam * lam;
-    const float planck = 1.19104297e-16f / (l2 * l2 * lam) / expm1f(a.q_c2_T * nu) * 1e-10f;
-    const int64_t n = a.n_v;
-    a.q_out[k] = A * a.q_path;
-    a.q_out[n + k] = eps;
-    a.q_out[2 * n + k] = 1.f - eps;
-    a.q_out[3 * n + k] = eps * planck;
-}
-
-template <int N1>
-__global__ void __launch_bounds__(ColShape<N1>::THREADS) k_col_ifft(const ColFftArgs a) {
-    constexpr int TPC = ColShape<N1>::TPC;
-    constexpr int B = ColShape<N1>::B;
-    extern __shared__ float2 sm[];
-    const int b = threadIdx.x % B;
-    const int j = threadIdx.x / B;
-    const int n2i = blockIdx.x * B + b;
-    float2 v[8];
-#pragma unroll
-    for (int q = 0; q < 8; ++q) v[q] = conjf2(a.h[(int64_t)(j + q * TPC) * a.n2 + n2i]);
-    col_fft8<N1>(v, sm, j, b, a.f1.tw);
-#pragma unroll
-    for (int r = 0; r < 8; ++r) {
-        const int64_t nidx = (int64_t)(j + r * TPC) * a.n2 + n2i;
-        if (nidx < a.n_v) {
-            const float A = v[r].x * a.out_scale;   // Re(conj(z)) = Re(z)
-            a.out[nidx] = A;
-            if (a.q_out) quantities_at(a, nidx, A);
-        }
-    }
-    // last kernel of the spectrum: hand the error flag to the host (mapped
-    // memory, read after the stream synchronises) and clear it
-    if (a.err_pub && blockIdx.x == 0 && threadIdx.x == 0) {
-        *a.err_pub = *a.err;
-        *a.err = 0u;
-    }
-}
-
-// ---------------------------------------------------------------------------
 // Derivatives with respect to (T, p, x), node axes held fixed.
 //
 // With the axes fixed the Voigt weights of the nodes are constants, so the
@@ -1593,38 +732,6 @@ __global__ void __launch_bounds__(ColShape<N1>::THREADS) k_col_ifft(const ColFft
 // in the real and node b in the imaginary part), and the per-line chain rule
 // gathers it back at each line's 8 cells (k_gather_grad).
 // ---------------------------------------------------------------------------
-
-// K2 on float rows: rows 2 pair and 2 pair + 1 of a.src, or (a.single) the
-// single row a.src with a zero partner.
-template <int N1>
-__global__ void __launch_bounds__(ColShape<N1>::THREADS) k_col_fft_fwd_f(const ColFftArgs a) {
-    constexpr int TPC = ColShape<N1>::TPC;
-    constexpr int B = ColShape<N1>::B;
-    extern __shared__ float2 sm[];
-    const int b = threadIdx.x % B;
-    const int j = threadIdx.x / B;
-    const int pair = blockIdx.y;
-    const float* ra = a.src + (a.single ? 0 : (int64_t)(2 * pair) * a.row_stride);
-    const float* rb = a.single ? nullptr : ra + a.row_stride;
-    const int n2i = blockIdx.x * B + b;
-    float2 v[8];
-#pragma unroll
-    for (int q = 0; q < 8; ++q) {
-        const int64_t nidx = (int64_t)(j + q * TPC) * a.n2 + n2i;
-        // buffer offset of FFT index nidx, or -1 where the row is zero
-        int64_t off = -1;
-        if (a.ext == 0) {
-            if (nidx < a.n_v) off = nidx;
-        } else if (nidx < a.n_v + a.ext) {
-            off = nidx + a.ext;
-        } else if (nidx >= a.n - a.ext) {
-            off = nidx - (a.n - a.ext);
-        }
-        v[q] = off >= 0 ? make_float2(__ldg(&ra[off]), rb ? __ldg(&rb[off]) : 0.f) : make_float2(0.f, 0.f);
-    }
-    col_fft8<N1>(v, sm, j, b, a.f1.tw);
-    store_twiddled<N1>(v, a, pair, j, n2i);
-}
 
 // Gaussian stage of the merged layout (see GaussArgs).  One CTA: one merged
 // row (wL node), kGaussTile consecutive outputs, kGaussPer per thread.  A merged row is
@@ -1853,69 +960,6 @@ __global__ void __launch_bounds__(128 * kSlitGroups) k_slit_conv(const SlitArgs 
     }
 }
 
-// Adjoint row stage, one CTA per (row k1, pair j): H = Ghat (V_2j + i V_2j+1)
-// on the row's bins k = k1 + n1 t, inverse row DFT, inverse four-step twiddle
-// w_N^{-t k1}; output y[j][k1][t].
-__global__ void __launch_bounds__(kRowThreads) k_row_ifft_adj(const AdjRowArgs a) {
-    extern __shared__ float2 sm[];
-    const VoigtArgs& v = a.v;
-    const int n2 = v.n2;
-    float2* buf0 = sm;
-    float2* buf1 = sm + row_buf_len(n2);
-    const int k1 = blockIdx.x;
-    const int j = blockIdx.y;
-    const int n = (int)v.n;
-    const NodeV A = node_params(v, 2 * j), B = node_params(v, 2 * j + 1);
-    const float2* gh = v.g + (int64_t)k1 * n2;
-    for (int t = threadIdx.x; t < n2; t += blockDim.x) {
-        const int kk = k1 + v.n1 * t;
-        const float f = (float)min(kk, n - kk) * v.inv_ndv;
-        const float va = voigt_eval(A, f, v.half_fs);
-        const float vb = voigt_eval(B, f, v.half_fs);
-        const float2 z = gh[t];
-        // inverse DFT = conj(forward DFT(conj(x)))
-        buf0[t] = make_float2(z.x * va - z.y * vb, -(z.y * va + z.x * vb));
-    }
-    __syncthreads();
-    bool padded;
-    const float2* res = fft_row(buf0, buf1, v.f2, &padded);
-    float2* y = a.y + ((int64_t)j * v.n1 + k1) * n2;
-    for (int t = threadIdx.x; t < n2; t += blockDim.x) {
-        float2 z = conjf2(res[padded ? rp(t) : t]);
-        if (k1 && t) z = cmul(z, conjf2(twiddle_n(v.tw_hi, v.tw_lo, t * k1)));
-        y[t] = z;
-    }
-}
-
-// Adjoint column stage: inverse column DFT (length n1) of pair `blockIdx.y`;
-// real part -> float row 2 pair, imaginary part -> row 2 pair + 1 of a.out
-// (first n_v samples, x out_scale).
-template <int N1>
-__global__ void __launch_bounds__(ColShape<N1>::THREADS) k_col_ifft_adj(const ColFftArgs a) {
-    constexpr int TPC = ColShape<N1>::TPC;
-    constexpr int B = ColShape<N1>::B;
-    extern __shared__ float2 sm[];
-    const int b = threadIdx.x % B;
-    const int j = threadIdx.x / B;
-    const int pair = blockIdx.y;
-    const int n2i = blockIdx.x * B + b;
-    const float2* h = a.h + (int64_t)pair * N1 * a.n2;
-    float2 v[8];
-#pragma unroll
-    for (int q = 0; q < 8; ++q) v[q] = conjf2(h[(int64_t)(j + q * TPC) * a.n2 + n2i]);
-    col_fft8<N1>(v, sm, j, b, a.f1.tw);
-    float* oa = a.out + (int64_t)(2 * pair) * a.row_stride;
-    float* ob = oa + a.row_stride;
-#pragma unroll
-    for (int r = 0; r < 8; ++r) {
-        const int64_t nidx = (int64_t)(j + r * TPC) * a.n2 + n2i;
-        if (nidx < a.n_v) {
-            oa[nidx] = v[r].x * a.out_scale;     // Re(conj(z))
-            ob[nidx] = -v[r].y * a.out_scale;    // Im(conj(z))
-        }
-    }
-}
-
 // Per-line derivative coefficients: dlnI/dtheta and the rates of the three
 // fractional coordinates, for theta = T, p_bar, x (radis/lbl/base.py:2664-2677
 // for I, broadening.py:170-172 and 368-381 for the widths, base.py:2351-2370
@@ -2075,49 +1119,11 @@ __global__ void __launch_bounds__(256) k_scatter_tangent(const GradArgs g) {
 static thread_local const char* g_launch_err = nullptr;
 const char* last_launch_error() { return g_launch_err; }
 
-static int check_launch() {
+int check_launch() {
     cudaError_t e = cudaGetLastError();
     g_launch_err = e == cudaSuccess ? nullptr : cudaGetErrorString(e);
     return e == cudaSuccess ? RG_OK : RG_ERR_CUDA;
 }
-
-int col_block(int n1) {
-    switch (n1) {
-        case 8: return ColShape<8>::B;
-        case 64: return ColShape<64>::B;
-        default: return ColShape<512>::B;
-    }
-}
-
-
-// Opt the kernel in to the largest dynamic shared memory the device allows
-// next to the kernel's own static shared memory; checks that `need` fits.
-// (first call per kernel: queries the attributes and sets the limit; later
-// calls only compare `need` with the cached limit)
-template <typename K>
-static int allow_smem(K kernel, std::atomic<size_t>& avail_cache, size_t need) {
-    size_t avail = avail_cache.load();
-    if (!avail) {
-        int dev = 0, optin = 0;
-        if (cudaGetDevice(&dev) != cudaSuccess) return RG_ERR_CUDA;
-        if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess)
-            return RG_ERR_CUDA;
-        cudaFuncAttributes fa;
-        if (cudaFuncGetAttributes(&fa, kernel) != cudaSuccess) return RG_ERR_CUDA;
-        avail = (size_t)optin - fa.sharedSizeBytes;
-        if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)avail) != cudaSuccess)
-            return RG_ERR_CUDA;
-        avail_cache.store(avail);
-    }
-    return need > avail ? RG_ERR_RANGE : RG_OK;
-}
-
-#define ALLOW_SMEM(kernel, need)                          \
-    do {                                                   \
-        static std::atomic<size_t> avail_{0};              \
-        int r_ = allow_smem(kernel, avail_, (need));       \
-        if (r_ != RG_OK) return r_;                        \
-    } while (0)
 
 int launch_prepare_lines(const double* v0_d, const double* s_d, int64_t n, double c2_tref, float2* v0_out,
                          float* ls2_out, int* unsorted_flag, cudaStream_t st) {
@@ -2181,134 +1187,6 @@ int scatter_smem_optin(size_t* avail, bool wide) {
     // every variant (and k_scatter_auto) has the same static shared memory
     // (none); the opt-in limit of one serves for all
     return wide ? scatter_optin<true>(avail) : scatter_optin<false>(avail);
-}
-
-template <int N1>
-static int col_fwd(const ColFftArgs& a, cudaStream_t st) {
-    ALLOW_SMEM(k_col_fft_fwd<N1>, N1 * ColShape<N1>::B * sizeof(float2));
-    dim3 grid(a.n2 / ColShape<N1>::B, a.n_pairs);
-    k_col_fft_fwd<N1><<<grid, ColShape<N1>::THREADS, N1 * ColShape<N1>::B * sizeof(float2), st>>>(a);
-    return check_launch();
-}
-
-int launch_col_fft_fwd(const ColFftArgs& a, cudaStream_t st) {
-    switch (a.n1) {
-        case 8: return col_fwd<8>(a, st);
-        case 64: return col_fwd<64>(a, st);
-        case 512: return col_fwd<512>(a, st);
-        default: return RG_ERR_RANGE;
-    }
-}
-
-template <int PAIRS, int MAXT, bool TWR, bool STAGE, bool TWS, bool SF>
-static int row_voigt(const VoigtArgs& a, cudaStream_t st) {
-    const size_t smem = row_voigt_smem<PAIRS>(a.n2, TWR, STAGE, TWS);
-    ALLOW_SMEM((k_row_fft_voigt<PAIRS, MAXT, TWR, STAGE, TWS, SF>), smem);
-    dim3 grid(a.n1, (a.n_pairs + kPairGroup - 1) / kPairGroup);
-    k_row_fft_voigt<PAIRS, MAXT, TWR, STAGE, TWS, SF><<<grid, a.threads, smem, st>>>(a);
-    return check_launch();
-}
-
-// Layout of the forward row kernel for rows of n2 points:
-//  * n2 <= 3072: two pairs per float4 element, <= 384 threads, the next two
-//    rows staged under the passes, and the per-row four-step twiddle table
-//    while two CTAs still fit an SM;
-//  * n2 <= 6144 (and the two work buffers fit): two pairs, <= 768 threads,
-//    one CTA per SM, nothing else in shared memory;
-//  * else one pair per element, <= 1024 threads.
-// Without the table the column stage applies the four-step twiddle.
-RowLayout row_layout(int n2) {
-    RowLayout L{};
-    if (n2 / 8 <= kRowMaxT2) {
-        L.pairs = 2;
-        L.maxt = kRowMaxT2;
-        L.stage = 1;
-        L.twr = row_voigt_smem<2>(n2, true, true) <= 113 * 1024;
-    } else if (n2 / 8 <= kRowMaxT2L && row_voigt_smem<2>(n2, false, false, true) <= 227 * 1024) {
-        L.pairs = 2;
-        L.maxt = kRowMaxT2L;
-    } else {
-        L.pairs = 1;
-        L.maxt = kRowMaxT1;
-    }
-    return L;
-}
-
-int launch_row_fft_voigt(const VoigtArgs& a, cudaStream_t st) {
-    if (a.f2.npass < 2 || a.f2.radix[a.f2.npass - 1] != 8) return RG_ERR_RANGE;
-    const RowLayout L = row_layout(a.n2);
-    if (a.threads < a.n2 / 8 || a.threads > L.maxt || a.threads % 32) return RG_ERR_RANGE;
-    if (L.pairs != a.pairs_per_pass || L.twr != a.row_twiddle_table) return RG_ERR_RANGE;
-    if (L.maxt == kRowMaxT2)
-        return L.twr ? row_voigt<2, kRowMaxT2, true, true, false, false>(a, st)
-                     : row_voigt<2, kRowMaxT2, false, true, false, false>(a, st);
-    if (L.maxt == kRowMaxT2L) return row_voigt<2, kRowMaxT2L, false, false, true, true>(a, st);
-    return row_voigt<1, kRowMaxT1, false, false, true, true>(a, st);
-}
-
-int launch_row_ifft(const RowIfftArgs& a, cudaStream_t st) {
-    const size_t smem = 2 * (size_t)row_buf_len(a.n2) * sizeof(float2);
-    ALLOW_SMEM(k_row_ifft, smem);
-    k_row_ifft<<<a.n1, kRowThreads, smem, st>>>(a);
-    return check_launch();
-}
-
-template <int N1>
-static int col_inv(const ColFftArgs& a, cudaStream_t st) {
-    ALLOW_SMEM(k_col_ifft<N1>, N1 * ColShape<N1>::B * sizeof(float2));
-    k_col_ifft<N1><<<a.n2 / ColShape<N1>::B, ColShape<N1>::THREADS, N1 * ColShape<N1>::B * sizeof(float2), st>>>(a);
-    return check_launch();
-}
-
-int launch_col_ifft(const ColFftArgs& a, cudaStream_t st) {
-    switch (a.n1) {
-        case 8: return col_inv<8>(a, st);
-        case 64: return col_inv<64>(a, st);
-        case 512: return col_inv<512>(a, st);
-        default: return RG_ERR_RANGE;
-    }
-}
-
-template <int N1>
-static int col_fwd_f(const ColFftArgs& a, cudaStream_t st) {
-    ALLOW_SMEM(k_col_fft_fwd_f<N1>, N1 * ColShape<N1>::B * sizeof(float2));
-    dim3 grid(a.n2 / ColShape<N1>::B, a.single ? 1 : a.n_pairs);
-    k_col_fft_fwd_f<N1><<<grid, ColShape<N1>::THREADS, N1 * ColShape<N1>::B * sizeof(float2), st>>>(a);
-    return check_launch();
-}
-
-int launch_col_fft_fwd_f(const ColFftArgs& a, cudaStream_t st) {
-    switch (a.n1) {
-        case 8: return col_fwd_f<8>(a, st);
-        case 64: return col_fwd_f<64>(a, st);
-        case 512: return col_fwd_f<512>(a, st);
-        default: return RG_ERR_RANGE;
-    }
-}
-
-int launch_row_ifft_adj(const AdjRowArgs& a, cudaStream_t st) {
-    const size_t smem = 2 * (size_t)row_buf_len(a.v.n2) * sizeof(float2);
-    ALLOW_SMEM(k_row_ifft_adj, smem);
-    dim3 grid(a.v.n1, a.v.n_pairs);
-    k_row_ifft_adj<<<grid, kRowThreads, smem, st>>>(a);
-    return check_launch();
-}
-
-template <int N1>
-static int col_inv_adj(const ColFftArgs& a, cudaStream_t st) {
-    ALLOW_SMEM(k_col_ifft_adj<N1>, N1 * ColShape<N1>::B * sizeof(float2));
-    dim3 grid(a.n2 / ColShape<N1>::B, a.n_pairs);
-    k_col_ifft_adj<N1><<<grid, ColShape<N1>::THREADS, N1 * ColShape<N1>::B * sizeof(float2), st>>>(a);
-    return check_launch();
-}
-
-int launch_col_ifft_adj(const ColFftArgs& a, cudaStream_t st) {
-    switch (a.n1) {
-        case 8: return col_inv_adj<8>(a, st);
-        case 64: return col_inv_adj<64>(a, st);
-        case 512: return col_inv_adj<512>(a, st);
-        default: return RG_ERR_RANGE;
-    }
 }
 
 // Row pitch of the projection coefficients: the rows rounded up to a multiple of 4.
@@ -2532,30 +1410,4 @@ int launch_scatter_tangent(const GradArgs& a, int grid, cudaStream_t st) {
     return check_launch();
 }
 
-}  // namespace rg
-
-namespace rg {
-// Thread count of the forward row kernel for a row plan: the multiple of 32
-// in [max(128, n2/8), layout limit] that wastes the fewest butterfly slots
-// over the passes (ties -> fewer threads).
-int row_threads(const FftLen& f) {
-    const int maxt = row_layout(f.L).maxt;
-    const int t_min = std::max(128, (f.L / 8 + 31) / 32 * 32);
-    int best = t_min;
-    double best_eff = -1.0;
-    for (int T = t_min; T <= maxt; T += 32) {
-        long slots = 0, work = 0;
-        for (int p = 0; p < f.npass; ++p) {
-            const int M = f.L / f.radix[p];
-            slots += (long)((M + T - 1) / T) * T;
-            work += M;
-        }
-        const double eff = (double)work / (double)slots;
-        if (eff > best_eff + 1e-9) {
-            best_eff = eff;
-            best = T;
-        }
-    }
-    return best;
-}
 }  // namespace rg

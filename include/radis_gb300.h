@@ -159,17 +159,16 @@ typedef struct {
      * and the half-width (points) of their widest Gaussian */
     int32_t fft_rows, merged_rows, merged_ext;
     float gauss_ms;            /* the real-space stage before the column FFT
-                                  (merged layout: the Gaussian stage; skeleton
-                                  layout: the projection), part of
+                                  (merged layout: the Gaussian stage), part of
                                   stage_ms[1] (timing = 1), else 0             */
     int32_t accum_bits;        /* the scatter's accumulator: 32 or 64 bits, or
                                   0 when it was chosen on the device (served
                                   and allocation-free spectra in auto mode)    */
     int32_t layout;            /* FFT-stage layout used: 1 node rows, 2 merged
-                                  rows, 3 skeleton rows (fft_rows of them)
-                                  projected in a pass of their own, 4 skeleton
-                                  rows projected by the scatter as it writes
-                                  each finished tile                           */
+                                  rows, 3 skeleton rows (fft_rows of them),
+                                  projected by the scatter as it writes each
+                                  finished tile, 4 the same on a grid of at
+                                  most 160 nodes                               */
     float layout_err;          /* skeleton layout: the largest error of the
                                   decomposition over its frequency samples     */
 } rg_spectrum_info;
@@ -304,10 +303,11 @@ int rg_slit_convolve(rg_ctx* ctx, const float* in_dev, int64_t n, const float* s
  * wait for copies already in flight always keeps the default bound. */
 int rg_plan_test_scatter_stall(rg_plan* plan, int32_t withhold, int64_t wait_cycles);
 
-/* Test hook, host-only, no counterpart in the reference: the node order in
- * which the scatter's flush projects a tile of n_nodes node rows on the tensor
- * cores (steps of 8 nodes: nodes[8 s + j]; real[8 s + j] = 0 where a node is
- * repeated with a zero coefficient).  *count = 8 x steps; RG_ERR_RANGE when
+/* Test hook, host-only, no counterpart in the reference: an order in which
+ * n_nodes tile rows with a pitch of 1 (mod 32) words are read eight at a time
+ * without bank conflicts (steps of 8 nodes: nodes[8 s + j]; real[8 s + j] = 0
+ * where a node is repeated with a zero coefficient).  The scatter's own tiles
+ * have a pitch that needs no order.  *count = 8 x steps; RG_ERR_RANGE when
  * capacity is smaller. */
 int rg_test_flush_order(int32_t n_nodes, int32_t* nodes, uint8_t* real, int32_t capacity, int32_t* count);
 

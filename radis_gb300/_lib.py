@@ -569,9 +569,9 @@ def grid_skeleton(grid: Grid, dv: float, folding_thresh: float = 1e-6, tol: floa
 
 
 def flush_order(n_nodes: int):
-    """Host-only test hook (rg_test_flush_order): the node order in which the
-    scatter's flush projects a tile on the tensor cores, as (nodes int32[8 S],
-    real bool[8 S]) for S steps of 8 nodes."""
+    """Host-only test hook (rg_test_flush_order): an order in which tile rows
+    of a pitch of 1 (mod 32) words are read eight at a time without bank
+    conflicts, as (nodes int32[8 S], real bool[8 S]) for S steps of 8 nodes."""
     cap = 8 * ((int(n_nodes) + 7) // 8 + 64)
     nodes = np.zeros(cap, np.int32)
     real = np.zeros(cap, np.uint8)

@@ -127,7 +127,8 @@ struct Envelope {
 struct rg_lines {
     rg_ctx* ctx = nullptr;
     int64_t n = 0;
-    float2* v0 = nullptr;
+    float* vh = nullptr;              // line centres as FP32 pairs (hi, lo)
+    float* vl = nullptr;
     float* ls2 = nullptr;
     float* el = nullptr;
     float* ga = nullptr;
@@ -193,7 +194,6 @@ struct Work {
     int skel_R = 0;
     double skel_err = 0.0;
     std::vector<int> skel_nodes;
-    int skel_flush_ks = 0;   // the scatter flush's tensor-core section: node steps (0: none)
     int last_accum = 0;               // accumulator bits of the last scatter (0: chosen on the device)
     int64_t row_stride = 0;
     float* ldm = nullptr;             // LDM [node][row_stride] (the scatter's float values)
@@ -682,63 +682,6 @@ int scatter_rng_cap(int64_t n_v, int sms) {
     return (cap + 1) & ~1;
 }
 
-// Lines per column from which the scatter keeps copies of a small tile.
-constexpr double kScatCopyDensity = 4.0;
-
-// Shape of the persistent scatter (one 1024-thread CTA per SM): TMA ring
-// stages, chunk (lines), tile width (columns), row pitch, copies of the tile
-// and dynamic shared memory, beside the line-range table (rng_cap entries) and
-// coef_bytes of skeleton projection data (0 without).
-struct ScatterShape {
-    int chunk = 0, TK = 0, pitch = 0, stages = 0, copies = 1, copy_words = 0;
-    size_t smem = 0;
-};
-int scatter_shape(int n_nodes, bool wide, size_t coef_bytes, int rng_cap, int64_t n_v, int sms, double lines_per_col,
-                  ScatterShape* sh) {
-    size_t avail = 0;
-    RG(scatter_smem_optin(&avail, wide));
-    const size_t word = wide ? 8 : 4;   // bytes per tile cell
-    auto tile_cols = [&](int S, int ch) {   // widest tile next to the ring (rows of tk + 1 words)
-        const size_t fixed = scatter_fixed_smem(ch, S, rng_cap) + coef_bytes + 16;
-        if (fixed >= avail) return 0;
-        return std::min(1024, ((int)((avail - fixed) / (word * (size_t)n_nodes)) - 1) / 32 * 32);
-    };
-    auto take = [&](int S, int ch, int tk_max) {
-        sh->chunk = ch;
-        sh->stages = S;
-        // the tiles of the fewest rounds of one tile per CTA, all equally wide:
-        // a window of few columns still reaches every SM (5001 columns, 2400
-        // lines each, 64-bit sums: 5 tiles of 1024 columns took 8.9 ms, 152 of 33
-        // take 0.18 ms), and the last round is full
-        const int64_t rounds = (n_v + (int64_t)sms * tk_max - 1) / ((int64_t)sms * tk_max);
-        const int64_t per = (n_v + rounds * sms - 1) / (rounds * sms);
-        sh->TK = (int)std::min<int64_t>(tk_max, per <= 64 ? per : (per + 15) / 16 * 16);
-        sh->pitch = (sh->TK + 31) / 32 * 32 + 1;
-        auto bytes = [&](int copies) {
-            return scatter_fixed_smem(ch, S, rng_cap) + coef_bytes +
-                   scatter_coef_offset((size_t)copies * scatter_copy_words(n_nodes, sh->pitch, wide, copies));
-        };
-        // copies of a small tile for lists of many lines per column: the lanes
-        // of a warp (sorted lines) then meet in one cell less often
-        sh->copies = 1;
-        while (lines_per_col >= kScatCopyDensity && sh->copies < 8 && bytes(2 * sh->copies) <= avail) sh->copies *= 2;
-        sh->copy_words = scatter_copy_words(n_nodes, sh->pitch, wide, sh->copies);
-        sh->smem = bytes(sh->copies);
-        return RG_OK;
-    };
-    // GB300 sweeps (CO2 5M / 128 nodes, H2O 100M / 288 nodes): one line per
-    // consumer thread per chunk (992 = 31 warps) in three stages while the tile
-    // keeps >= 192 columns (CO2 5M: 256 columns, or 224 beside the skeleton
-    // projection's 17 KB of tensor-core fragments, where three stages beat two
-    // 1536-line ones by 2%); else two 1536-line stages (wider tiles than 2048)
-    if (tile_cols(3, 992) >= 192) return take(3, 992, tile_cols(3, 992));
-    if (tile_cols(2, 1536) >= 64) return take(2, 1536, tile_cols(2, 1536));
-    for (int min_tk : {64, 32})
-        for (int ch : {1024, 512, 256})
-            if (tile_cols(2, ch) >= min_tk) return take(2, ch, tile_cols(2, ch));
-    return fail(RG_ERR_RANGE, "LDM grid of %d nodes does not fit a shared-memory tile", n_nodes);
-}
-
 // Mean lines per grid column of a list over its own range (all the host knows
 // of the density without reading the index back).
 double mean_lines_per_col(const rg_lines* L, double dv) {
@@ -751,13 +694,123 @@ double mean_lines_per_col(const rg_lines* L, double dv) {
     return (double)L->n * dv / std::max(span, dv);
 }
 
-// Shared-memory bytes of the skeleton projection beside the scatter's tile:
-// the tensor-core flush's section (32-bit tiles, where the grid has one) or
-// the FP32 coefficients.
-size_t fuse_smem_bytes(const ProjArgs* fuse, bool wide) {
-    if (!fuse) return 0;
-    if (!wide && fuse->flush) return flush_tc_bytes(fuse->flush_ks, fuse->flush_nr);
-    return sizeof(float) * (size_t)fuse->n_nodes * fuse->rows_pad;
+// Gaussian rows that a tile of `cols` columns needs at most: the cells of its
+// lines (the widest range of log v0 is the lowest tile's) and the row above.
+int tile_rows_needed(const rg_lines* L, const Work& W, const SpecHost& s, int cols) {
+    const rg_grid& g = s.grid;
+    double lo = std::numeric_limits<double>::infinity(), c_lo = lo, c_hi = -lo;
+    for (int i = 0; i < L->n_iso; ++i)
+        if (L->env.lv_min[i] <= L->env.lv_max[i]) {
+            lo = std::min(lo, L->env.lv_min[i]);
+            c_lo = std::min(c_lo, L->env.log_c2Mm[i]);
+            c_hi = std::max(c_hi, L->env.log_c2Mm[i]);
+        }
+    const double dv = W.desc.dv, margin = std::ceil(L->env.max_abs_delta * s.p_atm / dv) + 1;
+    const double v0 = std::max(W.desc.vmin - (margin + 1) * dv, std::exp(lo));
+    const double span = (std::log1p((cols + 2 * margin + 2) * dv / v0) + c_hi - c_lo) / g.dxG;
+    return span < g.n_G ? std::min(g.n_G, (int)(span + 0.2) + 3) : g.n_G;
+}
+
+// Lines per column from which the scatter keeps copies of a small tile.
+constexpr double kScatCopyDensity = 4.0;
+constexpr double kScatPeakDensity = 150.0;
+
+// Shape of the persistent scatter (one CTA per SM): TMA ring, line and flush
+// warps, tile width, rows, row pitch, copies and slots, and dynamic shared
+// memory.
+struct ScatterShape {
+    int line_warps = 0, chunk = 0, stages = 0, stage_bytes = 0;
+    int TK = 0, pitch = 0, win = 0, rows = 0, copies = 1, copy_words = 0, slots = 1;
+    bool frags = false;   // fused projection: coefficients in shared memory
+    size_t smem = 0;
+};
+int scatter_shape(const rg_lines* L, const Work& W, const SpecHost& s, bool wide, const ProjArgs* fuse, int rng_cap,
+                  ScatterShape* sh) {
+    size_t avail = 0;
+    RG(scatter_smem_optin(&avail, wide));
+    const int64_t n_v = W.desc.n_v;
+    const int sms = L->ctx->sms, NL = s.grid.n_L;
+    const size_t word = wide ? 8 : 4;   // bytes per tile cell
+    const double lines_per_col = mean_lines_per_col(L, W.desc.dv);
+    // the working warps shared out by the instructions per column of the two
+    // jobs: ~80 per 32 lines; a flush step of 8 nodes x 16 columns ~45 and its
+    // MMAs, or a store per node row.  Scatter over 7 / 9 / 11 / 13 / 15 / 17 /
+    // 19 line warps: 14.6 lines per column (5M) 70 / 64 / 60 / 59 / 58 / 68 / 75
+    // us, 67 (100M) 1063 / 968 / 834 / 858 / 816 / 799 / 856, 0.03 (10 000)
+    // 17.2 / 16.5 / 17.4 / 18.2 / 20 / 22 / 26
+    const int win256 = tile_rows_needed(L, W, s, 256);
+    const double flush = fuse ? ((win256 * NL + 7) / 8 * (40.0 + 6.0 * fuse->flush_nr) + 80.0) / 16.0 : 0.25 * s.n_nodes;
+    const double line = 2.5 * lines_per_col + 2.0;
+    constexpr double workers = kScatThreads / 32 - 1;
+    const int lw_best = std::max(9, std::min(19, ((int)(workers * line / (line + flush)) - 1) | 1));   // odd
+    // two copies of a tile where columns hold hundreds of lines (the densest
+    // one, where the host knows it)
+    const double peak = W.cmax_host >= 0 ? W.cmax_host / (2.0 * W.E) : lines_per_col;
+    int min_copies = !wide && fuse && peak >= kScatPeakDensity ? 2 : 1;
+    // the limit on a grid: a tile of all its nodes x 32 columns (+ 1) beside a ring of 256 lines
+    if (word * 33 * s.n_nodes + 2 * 33 * 256 + 80 + 8 * (size_t)rng_cap > avail)
+        return fail(RG_ERR_RANGE, "LDM grid of %d nodes does not fit a shared-memory tile", s.n_nodes);
+    // (tight: rows of 28 columns and the word beyond them in 32 words, without regard to banks)
+    auto fit = [&](int lw, int S, int slots, int min_tk, bool frags, bool tight) {
+        sh->line_warps = lw;
+        sh->chunk = 64 * lw;
+        sh->stage_bytes = sh->chunk * (28 + (L->dl ? 4 : 0) + (L->n_iso > 1 && L->iso ? 1 : 0));
+        sh->stages = S;
+        const size_t fixed = scatter_fixed_smem(sh->stage_bytes, S, rng_cap);
+        auto pitch_of = [&](int64_t tk) { return tight ? 32 : (int)((tk + 31) / 32 * 32 + 4); };
+        // the tile nodes' projection coefficients, 8 nodes x 8 rows in 512 bytes
+        sh->frags = fuse && frags;
+        auto frag_bytes = [&] { return sh->frags ? (size_t)sh->rows / 8 * fuse->flush_nr * 512 : 0; };
+        auto widest = [&](int slots_) {   // columns, a multiple of 32
+            const size_t cell = word * (size_t)sh->rows * slots_ * min_copies;
+            const size_t used = fixed + frag_bytes() + 64;
+            const int words = avail > used ? (int)((avail - used) / cell) : 0;   // of a tile row
+            return tight ? (words >= 32 ? 28 : 0) : std::max(0, std::min(1024, (words - 4) / 32 * 32));
+        };
+        int cols = 256;   // tile width that `win` covers
+        for (int it = 0; it < 4; ++it) {
+            sh->win = tile_rows_needed(L, W, s, cols);
+            sh->rows = (sh->win * NL + 7) / 8 * 8;
+            int tk = widest(slots);
+            sh->slots = slots;
+            if (n_v <= (int64_t)sms * widest(1)) {   // one tile per CTA
+                sh->slots = 1;
+                tk = widest(1);
+            }
+            if (tk < min_tk) return false;
+            // the tiles of the fewest rounds of one tile per CTA, all equally
+            // wide: a window of few columns still reaches every SM (5001
+            // columns, 2400 lines each, 64-bit sums: 5 tiles of 1024 columns
+            // took 8.9 ms, 152 of 33 take 0.18 ms), and the last round is full
+            const int64_t rounds = (n_v + (int64_t)sms * tk - 1) / ((int64_t)sms * tk);
+            const int64_t per = (n_v + rounds * sms - 1) / (rounds * sms);
+            sh->TK = (int)std::min<int64_t>(tk, per <= 64 ? per : (per + 15) / 16 * 16);
+            sh->pitch = pitch_of(sh->TK);
+            if (tile_rows_needed(L, W, s, sh->TK) <= sh->win) break;
+            if (it == 3) return false;
+            cols = it == 2 ? 1024 : sh->TK;
+        }
+        auto bytes = [&](int copies) {
+            const size_t w = (size_t)copies * scatter_copy_words(sh->rows, sh->pitch, wide, copies);
+            return fixed + (size_t)sh->slots * ((w + 3) / 4 * 16) + frag_bytes();
+        };
+        // copies of a small tile for lists of many lines per column: the lanes
+        // of a warp (sorted lines) then meet in one cell less often
+        sh->copies = min_copies;
+        while (lines_per_col >= kScatCopyDensity && n_v <= (int64_t)sms * sh->TK && sh->copies < 8 &&
+               bytes(2 * sh->copies) <= avail)
+            sh->copies *= 2;
+        sh->copy_words = scatter_copy_words(sh->rows, sh->pitch, wide, sh->copies);
+        sh->smem = bytes(sh->copies);
+        return sh->smem <= avail;
+    };
+    // two tiles of 64 columns or more; less; one tile; then (windows of some
+    // 500 nodes or more) without room for the projection's coefficients
+    if (fit(lw_best, 3, 2, 64, true, false) || fit(lw_best, 2, 2, 32, true, false) || fit(7, 2, 1, 32, true, false))
+        return RG_OK;
+    min_copies = 1;
+    if (fit(7, 2, 1, 32, true, false) || fit(7, 2, 1, 32, false, false) || fit(1, 2, 1, 28, false, true)) return RG_OK;
+    return fail(RG_ERR_RANGE, "LDM grid of %d nodes does not fit a shared-memory tile", s.n_nodes);
 }
 
 // fuse: the skeleton projection done by the scatter's flush (nullable); smem
@@ -766,7 +819,8 @@ int build_scatter_args(const rg_lines* L, const Work& W, const rg_conditions* c,
                        const ProjArgs* fuse, ScatterArgs* a, size_t* smem) {
     const rg_grid& g = s.grid;
     std::memset(a, 0, sizeof *a);
-    a->v0 = L->v0;
+    a->vh = L->vh;
+    a->vl = L->vl;
     a->ls2 = L->ls2;
     a->el = L->el;
     a->ga = L->ga;
@@ -783,28 +837,27 @@ int build_scatter_args(const rg_lines* L, const Work& W, const rg_conditions* c,
     a->NL = g.n_L;
     a->row_stride = W.row_stride;
     a->ldm = W.ldm;
-    const size_t coef_bytes = fuse_smem_bytes(fuse, wide);
     if (fuse) {
-        a->proj_coef = fuse->coef;
+        a->proj = fuse->flush;
         a->proj_rows = fuse->rows;
-        a->proj_rp = fuse->rows_pad;
-        a->n_real = fuse->n_nodes;
-        if (!wide && fuse->flush) {
-            a->proj_frag = fuse->flush;
-            a->proj_ks = fuse->flush_ks;
-            a->proj_nr = fuse->flush_nr;
-        }
+        a->proj_nr = fuse->flush_nr;
+        a->proj_np = fuse->flush_np;
     }
     a->rng_cap = scatter_rng_cap(W.desc.n_v, L->ctx->sms);
     ScatterShape sh;
-    RG(scatter_shape(s.n_nodes, wide, coef_bytes, a->rng_cap, W.desc.n_v, L->ctx->sms,
-                     mean_lines_per_col(L, W.desc.dv), &sh));
+    RG(scatter_shape(L, W, s, wide, fuse, a->rng_cap, &sh));
+    a->line_warps = sh.line_warps;
     a->chunk = sh.chunk;
+    a->stages = sh.stages;
+    a->stage_bytes = sh.stage_bytes;
     a->TK = sh.TK;
     a->pitch = sh.pitch;
-    a->stages = sh.stages;
+    a->win = sh.win;
+    a->rows = sh.rows;
     a->copies = sh.copies;
     a->copy_words = sh.copy_words;
+    a->slots = sh.slots;
+    a->proj_frags = sh.frags ? 1 : 0;
     if (smem) *smem = sh.smem;
     a->n_tiles = (int)((W.desc.n_v + a->TK - 1) / a->TK);
     a->cmax = W.cmax_dev;
@@ -841,6 +894,36 @@ int build_scatter_args(const rg_lines* L, const Work& W, const rg_conditions* c,
         split(b, &a->bI_hi[i], &a->bI_lo[i]);
     }
     a->stim_c = (float)(kC2 / T * kLog2e);
+    a->cG_lo = std::numeric_limits<float>::infinity();
+    a->cG_hi = -a->cG_lo;
+    for (int i = 0; i < L->n_iso; ++i)
+        if (L->env.lv_min[i] <= L->env.lv_max[i]) {
+            a->cG_lo = std::min(a->cG_lo, a->cG[i]);
+            a->cG_hi = std::max(a->cG_hi, a->cG[i]);
+        }
+    a->v_lo = (float)W.desc.vmin;
+    a->v_step = (float)W.desc.dv;
+    a->v_bot = (float)(std::exp(lv_lo) * (1.0 - 1e-6));
+    auto two = [](float x) { return float2{x, x}; };
+    LinePairs& k = a->k2;
+    k.neg_vmin_hi = two(-a->vmin_hi);
+    k.vmin_lo = two(a->vmin_lo);
+    k.inv_dv_hi = two(a->inv_dv_hi);
+    k.inv_dv_lo = two(a->inv_dv_lo);
+    k.p_atm = two(a->p_atm);
+    k.inv_vref = two(a->inv_vref);
+    k.lgG_scale = two(a->lgG_scale);
+    k.cG = two(a->cG[0]);
+    k.lgL_scale = two(a->lgL_scale);
+    k.tL = two(a->tL);
+    k.cL = two(a->cL);
+    k.x_self = two(a->x_self);
+    k.aT_hi = two(a->aT_hi);
+    k.aT_lo = two(a->aT_lo);
+    k.bI_hi = two(a->bI_hi[0]);
+    k.bI_lo = two(a->bI_lo[0]);
+    k.stim = two(a->stim_c);
+    k.n_l = two((float)g.n_L);
     a->in_window = W.count_lines ? W.counter : nullptr;
     a->wait_limit = W.scat_wait;
     a->withhold = W.scat_withhold;
@@ -1056,13 +1139,8 @@ int NL_merged(const GaussArgs& ga) { return ga.NLv; }
 // every node's transform within tol; fills the row kernel's arguments (row r
 // = skeleton node sk[r], with its own transform) and the projection
 // coefficients [n_nodes][rows_pad] in W.proj_host.
-// Skeleton projection in the scatter's flush (no LDM round trip through HBM)
-// for grids of at most this many nodes; larger grids project in a separate
-// pass, with the decomposition computed on the host while the scatter runs.
-// Measured on the 288-node H2O 100M grid, also with a tensor-core flush of
-// three row blocks: its fragments leave 64-column tiles (4 flush tasks for 31
-// warps) and the fused scatter took 1.91 ms against 1.13 + 0.41 ms for the
-// scatter and the pass.
+// The scatter projects each finished tile onto the skeleton rows as it writes
+// it.  Grids of more nodes report layout 3, smaller ones 4 (rg_spectrum_info).
 constexpr int kFuseMaxNodes = 160;
 
 constexpr int kSkelSamples = 32;
@@ -1126,14 +1204,14 @@ int skeleton_decomp(const rg_grid& g, double dv, double thresh, double tol, int 
     return interp_decomp(A.data(), S, n, tol, r_max, sk->data(), C->data(), R, err);
 }
 
-// Node order of the scatter flush's tensor-core form (steps of 8 nodes, see
-// flush_tc): tile rows have a pitch of 1 (mod 32) words, so node m sits in the
-// bank class m mod 32 = 8 ((m / 8) mod 4) + m mod 8, and the four nodes that
-// one A-fragment load reads (t = 0..3) must come from the classes v, v + 8,
-// v + 16, v + 24.  Nodes are grouped by (m mod 8, (m / 8) mod 4) into such
-// quadruples; a class short of nodes repeats one of its nodes (real = 0: a
-// zero coefficient), two quadruples make a step.  Below 32 nodes some classes
-// are empty and no order is conflict-free: the natural one, padded.
+// Order in which nodes of tile rows with a pitch of 1 (mod 32) words are read
+// eight at a time without bank conflicts (the scatter's own tiles have a pitch
+// of 4 (mod 32), where every order is free of them): node m sits in the bank
+// class m mod 32 = 8 ((m / 8) mod 4) + m mod 8, and the four nodes of one load
+// must come from the classes v, v + 8, v + 16, v + 24.  Nodes are grouped by
+// (m mod 8, (m / 8) mod 4) into such quadruples; a class short of nodes repeats
+// one of its nodes (real = 0), two quadruples make a step.  Below 32 nodes some
+// classes are empty and no order is conflict-free: the natural one, padded.
 void flush_node_order(int n, std::vector<int>* nodes, std::vector<char>* real) {
     nodes->clear();
     real->clear();
@@ -1188,7 +1266,6 @@ bool plan_skeleton(Work& W, const SpecHost& s, const VoigtArgs& va, int r_max, V
         std::copy(key, key + 10, W.skel_key);
         W.skel_valid = true;
         W.skel_R = 0;   // no skeleton layout for this grid (cached as well)
-        W.skel_flush_ks = 0;
         std::vector<int> sk;
         std::vector<double> C;
         int R = 0;
@@ -1197,26 +1274,21 @@ bool plan_skeleton(Work& W, const SpecHost& s, const VoigtArgs& va, int r_max, V
         const int rows = R + (R & 1);
         if (R < 1 || rows > r_max) return false;
         const int rp = proj_rows_pad(rows);
-        // coefficients in shared memory: beside the scatter's tile (grids of up
-        // to kFuseMaxNodes nodes) or as the projection pass's fragments
+        // limits of the derivatives' kernels: the adjoint's gather and the
+        // tangents' projection pass keep the coefficients in shared memory
         if ((size_t)n * rp * sizeof(float) > 96 * 1024) return false;
         if (n > kFuseMaxNodes && proj_tc_smem((rows + 7) / 8, 2 * ((n + 15) / 16)) > kProjTcSmemMax) return false;
-        // [n][rp] coefficients (the FP32 forms), then the tensor-core pass's B
-        // fragments: TF32 hi / lo parts, [nr][ks][part][lane][2] with
+        // [n][rp] coefficients (the gather); the projection pass's B
+        // fragments (neither on the allocation-free path): TF32 hi / lo parts, [nr][ks][part][lane][2] with
         // b0, b1 = C[8 nr + g][8 ks + t], C[8 nr + g][8 ks + t + 4], g = lane / 4,
-        // t = lane % 4
-        const int NR = (rows + 7) / 8, KSP = 2 * ((n + 15) / 16);
-        // the scatter flush's tensor-core section (fused grids of up to two
-        // row blocks): B fragments [ks][nr][lane] (b0, b1 hi, b0, b1 lo) in
-        // the flush's node order, then that order as a table [ks][t][2]
-        std::vector<int> fl_nodes;
-        std::vector<char> fl_real;
-        if (n <= kFuseMaxNodes && NR <= 2) flush_node_order(n, &fl_nodes, &fl_real);
-        const int KSF = (int)fl_nodes.size() / 8;
-        W.proj_host.assign((size_t)n * rp + (size_t)NR * KSP * 128 + flush_tc_bytes(KSF, NR) / sizeof(float), 0.f);
+        // t = lane % 4; the scatter's flush: (hi, lo) [nr][n + 8][8]
+        const int NR = (rows + 7) / 8, KSP = W.proj_fixed ? 0 : 2 * ((n + 15) / 16);
+        const size_t np = n + 8, coefs = W.proj_fixed ? 0 : (size_t)n * rp;
+        W.proj_host.assign(coefs + (size_t)NR * KSP * 128 + (size_t)NR * np * 16, 0.f);
         for (int r = 0; r < R; ++r)
-            for (int node = 0; node < n; ++node) W.proj_host[(size_t)node * rp + r] = (float)C[(size_t)r * n + node];
-        float* fr = W.proj_host.data() + (size_t)n * rp;
+            for (int node = 0; node < n && coefs; ++node)
+                W.proj_host[(size_t)node * rp + r] = (float)C[(size_t)r * n + node];
+        float* fr = W.proj_host.data() + coefs;
         auto cf = [&](int r, int k) { return r < R && k < n ? (float)C[(size_t)r * n + k] : 0.f; };
         for (int nr = 0; nr < NR; ++nr)
             for (int ks = 0; ks < KSP; ++ks)
@@ -1230,34 +1302,25 @@ bool plan_skeleton(Work& W, const SpecHost& s, const VoigtArgs& va, int r_max, V
                     }
                 }
         float* ff = fr + (size_t)NR * KSP * 128;
-        for (int ks = 0; ks < KSF; ++ks)
-            for (int nr = 0; nr < NR; ++nr)
-                for (int lane = 0; lane < 32; ++lane) {
-                    const int g = lane >> 2, t = lane & 3;
-                    float* o = ff + ((size_t)(ks * NR + nr) * 32 + lane) * 4;
-                    for (int i = 0; i < 2; ++i) {
-                        const int j = 8 * ks + t + 4 * i;
-                        const float v = fl_real[j] ? cf(8 * nr + g, fl_nodes[j]) : 0.f;
-                        o[i] = tf32_round_host(v);
-                        o[2 + i] = tf32_round_host(v - o[i]);
-                    }
-                }
-        int32_t* tbl = reinterpret_cast<int32_t*>(ff + (size_t)KSF * NR * 128);
-        for (int ks = 0; ks < KSF; ++ks)
-            for (int t = 0; t < 4; ++t) {
-                tbl[ks * 8 + 2 * t] = fl_nodes[8 * ks + t];
-                tbl[ks * 8 + 2 * t + 1] = fl_nodes[8 * ks + t + 4];
+        for (int r = 0; r < R; ++r)
+            for (int node = 0; node < n; ++node) {
+                float* o = ff + (((size_t)(r / 8) * np + node) * 8 + r % 8) * 2;
+                const float v = (float)C[(size_t)r * n + node];
+                o[0] = tf32_round_host(v);
+                o[1] = tf32_round_host(v - o[0]);
             }
-        W.skel_flush_ks = KSF;
         W.skel_nodes.assign(sk.begin(), sk.begin() + R);
         W.skel_R = R;
         W.skel_err = err;
     }
     if (W.skel_R == 0) return false;
-    if (W.proj_fixed && sizeof(float) * W.proj_host.size() > W.proj_bytes) return false;
     const int R = W.skel_R;
     const int rows = R + (R & 1);
     const int rp = proj_rows_pad(rows);
+    // the allocation-free path's limit: coefficients and two fragments of 16 nodes in 256 KB
+    if (W.proj_fixed && (sizeof(float) * (size_t)n * rp + (size_t)((rows + 7) / 8) * ((n + 15) / 16) * 1024 > 256 * 1024 ||
+                         sizeof(float) * W.proj_host.size() > W.proj_bytes))
+        return false;
     const double err = W.skel_err;
     const std::vector<int>& sk = W.skel_nodes;
     *vk = va;
@@ -1289,9 +1352,9 @@ bool plan_skeleton(Work& W, const SpecHost& s, const VoigtArgs& va, int r_max, V
     pa->rows = rows;
     pa->rows_pad = rp;
     pa->mtiles = (rows + 7) / 8;   // the tensor-core pass's 8-row n-tiles
-    pa->ksteps = 2 * ((n + 15) / 16);
-    pa->flush_ks = W.skel_flush_ks;
-    pa->flush_nr = W.skel_flush_ks ? pa->mtiles : 0;
+    pa->ksteps = W.proj_fixed ? 0 : 2 * ((n + 15) / 16);
+    pa->flush_nr = pa->mtiles;
+    pa->flush_np = n + 8;
     *err_out = err;
     return true;
 }
@@ -1309,15 +1372,13 @@ int take_err(Work& W) {
 // stages (unless ldm_only), and the publication of the device error flag.
 // ev: 6 events recorded between stages (nullable).
 // Shape of the scatter with the 32- or 64-bit accumulator: arguments, grid
-// (one persistent CTA per SM, more only past kScatMaxTilesPerCta tiles each)
+// (one persistent CTA per SM, more only past rng_cap tiles each)
 // and dynamic shared memory.
 int scatter_launch_shape(const rg_lines* L, const Work& W, const rg_conditions* c, const SpecHost& s, bool wide,
                          const ProjArgs* fuse, ScatterArgs* sa, int* grid, size_t* smem) {
     RG(build_scatter_args(L, W, c, s, wide, fuse, sa, smem));
     const int sms = L->ctx->sms;
-    *grid = std::max(std::min(sa->n_tiles, sms), (sa->n_tiles + kScatMaxTilesPerCta - 1) / kScatMaxTilesPerCta);
-    if ((sa->n_tiles + *grid - 1) / *grid > sa->rng_cap)
-        return fail(RG_ERR_RANGE, "scatter tiles per CTA above the line-range table");
+    *grid = std::max(std::min(sa->n_tiles, sms), (sa->n_tiles + sa->rng_cap - 1) / sa->rng_cap);
     return RG_OK;
 }
 
@@ -1375,10 +1436,11 @@ int plan_layout(Work& W, const SpecHost& s, cudaStream_t st, LayoutPlan* lp) {
             W.skel_dev = true;
         }
         lp->pa.coef = W.proj_coef;
-        // the tensor-core fragments follow the [n][rp] coefficients, then the
-        // scatter flush's section
-        lp->pa.frag = W.proj_coef + (size_t)lp->pa.n_nodes * lp->pa.rows_pad;
-        lp->pa.flush = lp->pa.flush_ks ? lp->pa.frag + (size_t)lp->pa.mtiles * lp->pa.ksteps * 128 : nullptr;
+        // the projection pass's fragments follow the [n][rp] coefficients, then
+        // the scatter flush's section (the allocation-free path has it alone)
+        lp->pa.frag = W.proj_coef + (W.proj_fixed ? 0 : (size_t)lp->pa.n_nodes * lp->pa.rows_pad);
+        lp->pa.flush =
+            reinterpret_cast<const float2*>(lp->pa.frag + (size_t)lp->pa.mtiles * lp->pa.ksteps * 128);
     }
     return RG_OK;
 }
@@ -1390,13 +1452,9 @@ int enqueue_spectrum(const rg_lines* L, Work& W, const rg_conditions* c, const S
     const int n_v = (int)W.desc.n_v;
     const int n_real = s.grid.n_G * s.grid.n_L;
     LayoutPlan lp;
-    bool planned = false;
-    if (!ldm_only && W.allow_skeleton && (W.desc.layout == 0 || W.desc.layout == 3) && n_real <= kFuseMaxNodes) {
-        RG(plan_layout(W, s, st, &lp));
-        planned = true;
-    }
+    if (!ldm_only) RG(plan_layout(W, s, st, &lp));
     lp.pa.sms = L->ctx->sms;
-    const ProjArgs* fuse = planned && lp.skel ? &lp.pa : nullptr;
+    const ProjArgs* fuse = !ldm_only && lp.skel ? &lp.pa : nullptr;
     if (ev) CU(cudaEventRecord(ev[0], st));
     if (W.count_lines) CU(cudaMemsetAsync(W.counter, 0, sizeof(unsigned long long), st));
     // accumulator width: forced, or from the densest column when the host knows
@@ -1418,7 +1476,7 @@ int enqueue_spectrum(const rg_lines* L, Work& W, const rg_conditions* c, const S
         RG(launch_scatter_auto(a32, a64, std::max(g32, g64), kScatThreads, std::max(m32, m64), st));
         W.last_accum = 0;
     }
-    if (fuse) W.last_layout = 4;
+    if (fuse && n_real <= kFuseMaxNodes) W.last_layout = 4;
     if (ev) CU(cudaEventRecord(ev[1], st));
     if (!ldm_only) {
         ColFftArgs ca;
@@ -1434,15 +1492,10 @@ int enqueue_spectrum(const rg_lines* L, Work& W, const rg_conditions* c, const S
         ca.y = W.y;
         ca.tw_hi = W.tw_hi;
         ca.tw_lo = W.tw_lo;
-        if (!planned) {
-            RG(plan_layout(W, s, st, &lp));
-            lp.pa.sms = L->ctx->sms;
-        }
         const bool skel = lp.skel, merged = lp.merged;
         GaussArgs* ga = lp.ga.get();
         ProjArgs& pa = lp.pa;
         if (skel) {
-            if (!fuse) RG(launch_node_project(pa, st));
             if (ev) CU(cudaEventRecord(ev[6], st));
             ca.n_pairs = pa.rows / 2;
             RG(launch_col_fft_fwd(ca, st));
@@ -1857,7 +1910,8 @@ int rg_lines_upload(rg_ctx* ctx, const rg_line_arrays* in, const rg_isotopes* is
     };
     auto bail = [&](int code) {
         cleanup_tmp();
-        dfree(L->v0);
+        dfree(L->vh);
+        dfree(L->vl);
         dfree(L->ls2);
         dfree(L->el);
         dfree(L->ga);
@@ -1881,7 +1935,8 @@ int rg_lines_upload(rg_ctx* ctx, const rg_line_arrays* in, const rg_isotopes* is
     CUB(cudaMalloc(&v0_tmp, sizeof(double) * n));
     CUB(cudaMalloc(&s_tmp, sizeof(double) * n));
     CUB(cudaMalloc(&flag, sizeof(int)));
-    CUB(cudaMalloc(&L->v0, sizeof(float2) * npad));
+    CUB(cudaMalloc(&L->vh, f4p));
+    CUB(cudaMalloc(&L->vl, f4p));
     CUB(cudaMalloc(&L->ls2, f4p));
     CUB(cudaMalloc(&L->el, f4p));
     CUB(cudaMalloc(&L->ga, f4p));
@@ -1891,8 +1946,7 @@ int rg_lines_upload(rg_ctx* ctx, const rg_line_arrays* in, const rg_isotopes* is
     if (in->iso && L->n_iso > 1) CUB(cudaMalloc(&L->iso, (size_t)npad));
     if (npad > n) {   // padding lines: v0 = 0 lies outside every window and is dropped
         const int64_t t = npad - n;
-        CUB(cudaMemsetAsync(L->v0 + n, 0, sizeof(float2) * t, st));
-        for (float* arr : {L->ls2, L->el, L->ga, L->gs, L->na, L->dl})
+        for (float* arr : {L->vh, L->vl, L->ls2, L->el, L->ga, L->gs, L->na, L->dl})
             if (arr) CUB(cudaMemsetAsync(arr + n, 0, sizeof(float) * t, st));
         if (L->iso) CUB(cudaMemsetAsync(L->iso + n, 0, (size_t)t, st));
     }
@@ -1905,7 +1959,7 @@ int rg_lines_upload(rg_ctx* ctx, const rg_line_arrays* in, const rg_isotopes* is
     CUB(cudaMemcpyAsync(L->na, in->n_air, f4, cudaMemcpyHostToDevice, st));
     if (in->delta) CUB(cudaMemcpyAsync(L->dl, in->delta, f4, cudaMemcpyHostToDevice, st));
     if (L->iso) CUB(cudaMemcpyAsync(L->iso, in->iso, (size_t)n, cudaMemcpyHostToDevice, st));
-    if (launch_prepare_lines(v0_tmp, s_tmp, n, kC2 / L->t_ref, L->v0, L->ls2, flag, st) != RG_OK)
+    if (launch_prepare_lines(v0_tmp, s_tmp, n, kC2 / L->t_ref, L->vh, L->vl, L->ls2, flag, st) != RG_OK)
         return bail(fail(RG_ERR_CUDA, "prepare_lines launch: %s", cudaGetErrorString(cudaGetLastError())));
     int unsorted = 0;
     CUB(cudaMemcpyAsync(&unsorted, flag, sizeof(int), cudaMemcpyDeviceToHost, st));
@@ -1929,7 +1983,8 @@ int rg_lines_free(rg_lines* L) {
     DeviceGuard dev_guard_;
     dev_guard_.use(L->ctx->device);
     cudaStreamSynchronize(L->ctx->stream);
-    dfree(L->v0);
+    dfree(L->vh);
+    dfree(L->vl);
     dfree(L->ls2);
     dfree(L->el);
     dfree(L->ga);
@@ -1986,7 +2041,7 @@ int rg_plan_create(rg_lines* L, const rg_plan_desc* d, rg_plan** out) {
     W.col_count = (int)d->n_v + 1 + 2 * W.E;
     cudaStream_t st = L->ctx->stream;
     CU(cudaMalloc(&W.col_start, sizeof(int64_t) * W.col_count));
-    RG(launch_col_index(L->v0, L->n, d->vmin, d->dv, -W.E, W.col_count, W.col_start, st));
+    RG(launch_col_index(L->vh, L->vl, L->n, d->vmin, d->dv, -W.E, W.col_count, W.col_start, st));
     CU(cudaMalloc(&W.cmax_dev, sizeof(int)));
     RG(launch_col_cmax(W.col_start, W.col_off, W.col_count, (int)d->n_v, W.E - 1, W.cmax_dev, st));
     W.row_stride = (d->n_v + 31) / 32 * 32;
@@ -2605,7 +2660,7 @@ int start_on_slot(rg_server* S, int si, const std::shared_ptr<ServerReq>& r, con
         sl.pin_cap = cap;
     }
     const rg_lines* L = r->lines;
-    RG(launch_col_index(L->v0, L->n, d.vmin, d.dv, -W.E, W.col_count, W.col_start, sl.st));
+    RG(launch_col_index(L->vh, L->vl, L->n, d.vmin, d.dv, -W.E, W.col_count, W.col_start, sl.st));
     RG(launch_col_cmax(W.col_start, W.col_off, W.col_count, (int)d.n_v, W.E - 1, W.cmax_dev, sl.st));
     RG(enqueue_spectrum(L, W, &r->cond, sh, direct ? direct : sl.out_d, sl.st, nullptr, false));
     if (!direct)
@@ -3002,8 +3057,8 @@ extern "C" int rg_synthesize_static(rg_lines* L, const rg_plan_desc* d, const rg
     W.tw_lo = twl;
     // sized here: the workspace step finds them large enough and allocates nothing;
     // the merged layout (its own row buffer) is not used on this path; the
-    // skeleton layout's coefficients get a fixed piece (the largest a grid can
-    // need: [n][rp] <= 96 KB plus tensor-core fragments < 150 KB)
+    // skeleton layout's coefficients get a fixed piece (more than plan_skeleton's
+    // limit leaves a grid)
     W.allow_merge = false;
     W.allow_skeleton = true;
     W.proj_fixed = true;
@@ -3037,7 +3092,7 @@ extern "C" int rg_synthesize_static(rg_lines* L, const rg_plan_desc* d, const rg
     RG(static_twiddles(W.f2.tw, W.n2, W.n2, 1, st));
     RG(static_twiddles(twh, nh, W.n, 1024, st));
     RG(static_twiddles(twl, 1024, W.n, 1, st));
-    RG(launch_col_index(L->v0, L->n, d->vmin, d->dv, -W.E, W.col_count, W.col_start, st));
+    RG(launch_col_index(L->vh, L->vl, L->n, d->vmin, d->dv, -W.E, W.col_count, W.col_start, st));
     RG(launch_col_cmax(W.col_start, W.col_off, W.col_count, (int)d->n_v, W.E - 1, W.cmax_dev, st));
     RG(enqueue_spectrum(L, W, c, s, out_dev, st, nullptr, false));
     drain.armed = false;

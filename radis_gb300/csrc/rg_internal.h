@@ -111,8 +111,17 @@ struct FftLen {
 };
 
 // --- kernel argument blocks (passed by value) ----------------------------------
+// The per-line constants of a ScatterArgs, each in both lanes of a packed pair
+// (the scatter works on two lines per thread).
+struct LinePairs {
+    float2 neg_vmin_hi, vmin_lo, inv_dv_hi, inv_dv_lo, p_atm;
+    float2 inv_vref, lgG_scale, cG, lgL_scale, tL, cL, x_self;
+    float2 aT_hi, aT_lo, bI_hi, bI_lo, stim;
+    float2 n_l;               // NL
+};
 struct ScatterArgs {
-    const float2* v0;     // (hi, lo) split of the FP64 line centre
+    const float* vh;      // (hi, lo) split of the FP64 line centre
+    const float* vl;
     const float* ls2;     // log2 S_ref - log2(1 - exp(-c2 v0 / Tref))
     const float* el;
     const float* ga;
@@ -124,10 +133,6 @@ struct ScatterArgs {
     int col_off;
     int col_count;
     int n_v;
-    int TK;               // columns per tile
-    int pitch;            // words per tile row: 1 (mod 32), >= TK + 1
-    int copies;           // copies of the tile (1, 2, 4 or 8): lane l adds into copy l mod copies
-    int copy_words;       // words from one copy to the next
     int n_nodes;          // padded to even
     int NG, NL;
     int64_t row_stride;
@@ -146,65 +151,68 @@ struct ScatterArgs {
     float aT_hi, aT_lo;       // -c2 (1/T - 1/Tref) log2e (double-float)
     float bI_hi[kMaxIso], bI_lo[kMaxIso];   // (log(Qr N x) - log_scale) log2e
     float stim_c;             // c2/T log2e
+    LinePairs k2;             // the above (isotopologue 0) in pairs
     unsigned long long* in_window;   // nullable counter of lines in the window
+    // tile of a CTA (rg_kernels.cu): the grid nodes of `win` Gaussian rows that
+    // the tile's lines can reach, from row l_base(tile) on
+    int TK;                   // columns per tile
+    int pitch;                // words per tile row: 4 (mod 32) (32 where the tile is tight), > TK
+    int win;                  // Gaussian rows of the tile (2 .. NG)
+    int rows;                 // tile rows: win x NL rounded up to 8
+    int copies;               // copies of the tile (1, 2, 4 or 8): lane l adds into copy l mod copies
+    int copy_words;           // words from one copy to the next
+    int slots;                // tiles in flight (1 or 2)
+    float cG_lo, cG_hi;       // smallest and largest cG
+    float v_lo, v_step, v_bot;   // v0 of column c is v_lo + c v_step; the list starts above v_bot
     // persistent TMA-fed scatter
     const int* cmax;          // device: most lines that can touch one column (sets the fixed-point scale)
     int n_tiles;
-    int chunk;                // lines per staged chunk (multiple of 16)
+    int chunk;                // lines per staged chunk: 64 per line warp
     int stages;               // chunk buffers in the TMA ring (2..kScatMaxStages)
+    int stage_bytes;
+    int line_warps;           // odd; the other warps but the producer flush
     unsigned* err;            // set to 1 when a bounded wait gives up
     long long wait_limit;     // SM clock cycles a producer/consumer handshake wait may take
     int withhold;             // test hook: the producer issues no line copies, so the
                               // consumers' waits run out (the error path, exercised safely)
-    // skeleton layout fused into the flush (proj_coef non-null): each finished
-    // tile is written as proj_rows skeleton rows (ldm rows [0, proj_rows)),
-    // row r = sum over the n_real node rows of proj_coef[node * proj_rp + r] x row
-    const float* proj_coef;   // [n_real][proj_rp], staged into shared memory after the tile
+    // skeleton layout (proj non-null): each finished tile is written as
+    // proj_rows skeleton rows (ldm rows [0, proj_rows)), row r = sum over the
+    // node rows of C[node][r] x row; proj: (hi, lo) TF32 parts of C, [row
+    // block of 8][proj_np nodes][8], zero from the n-th node on
+    const float2* proj;
     int proj_rows;            // even; rows >= the skeleton's are zero rows
-    int proj_rp;              // coefficient pitch, a multiple of 4
-    int n_real;               // NG x NL (the pad node of an odd grid is not read)
-    // tensor-core form of that flush (32-bit tiles; nullable): B fragments
-    // [proj_ks][proj_nr][32] x 4 floats (b0, b1 TF32 hi, then lo), then the
-    // node table [proj_ks][8] ints (step s: node(s, t), node(s, t + 4) for
-    // t = 0..3)
-    const float* proj_frag;
-    int proj_ks;              // node steps of 8
-    int proj_nr;              // row blocks of 8 (1 or 2)
+    int proj_nr;              // row blocks of 8
+    int proj_np;              // nodes, with at least 8 of padding
+    int proj_frags;           // 1: the tile's part of proj is kept in shared memory
     int rng_cap;              // entries of the per-tile line-range table (>= tiles per CTA, even)
 };
 constexpr long long kScatWaitCycles = 1LL << 31;   // about one second of SM clocks
 
-// Lines are staged per chunk as [v0 8B][ls2][el][ga][gs][na][dl 4B each][iso 1B]
-// x chunk; line arrays are allocated with room for a multiple of 16 lines.
+// Lines are staged per chunk as [vh][vl][ls2][el][ga][gs][na][dl 4B each][iso
+// 1B] x chunk; line arrays are allocated with room for a multiple of 16 lines.
 constexpr int kLinePad = 16;
-constexpr int kScatThreads = 1024;
+constexpr int kScatThreads = 768;
 constexpr int kScatMaxTilesPerCta = 512;
 #ifdef __CUDACC__
 #define RG_HD __host__ __device__
 #else
 #define RG_HD
 #endif
-constexpr int kScatMaxStages = 4;
-RG_HD inline size_t scatter_stage_bytes(int chunk) { return (size_t)33 * chunk; }
-// bytes of the tensor-core flush's fragments and node table in shared memory
-RG_HD inline size_t flush_tc_bytes(int ks, int nr) { return (size_t)ks * nr * 512 + (size_t)ks * 32; }
-// stage ring, its full and empty mbarriers (one 64-byte block) and the
-// per-tile line ranges (rng_cap entries of 8 bytes, rng_cap even: the tile
-// after them starts on a 16-byte boundary)
-RG_HD inline size_t scatter_fixed_smem(int chunk, int stages, int rng_cap) {
-    return stages * scatter_stage_bytes(chunk) + 16 * kScatMaxStages + 8 * (size_t)rng_cap;
+constexpr int kScatMaxStages = 8;
+// the ring, its full and empty mbarriers, the tile slots' full and free ones and
+// the flush warps' own (one 192-byte block), the per-tile line ranges (rng_cap entries of 8 bytes,
+// rng_cap even) and the 16 bytes before the first tile that a line one column
+// left of it writes
+RG_HD inline size_t scatter_fixed_smem(int stage_bytes, int stages, int rng_cap) {
+    return (size_t)stages * stage_bytes + 192 + 8 * (size_t)rng_cap + 16;
 }
-// 32-bit words of one copy of a tile of n_nodes rows (64-bit accumulator: the
-// low words' plane, then the high words'); copies beyond the first start 4
-// words (mod 32) further, so that the same cell of the eight copies lies in
-// eight distinct groups of four banks
-RG_HD inline int scatter_copy_words(int n_nodes, int pitch, bool wide, int copies) {
-    const int w = n_nodes * pitch * (wide ? 2 : 1);
-    return copies > 1 ? (w - 4 + 31) / 32 * 32 + 4 : w;
+// 32-bit words of one copy of a tile (64-bit accumulator: the low words'
+// plane, then the high words').  Copies start 1 word (mod 32) further each:
+// rows are 4 (mod 32) apart, so the cells of one column spread over all banks.
+RG_HD inline int scatter_copy_words(int rows, int pitch, bool wide, int copies) {
+    const int w = rows * pitch * (wide ? 2 : 1);
+    return copies > 1 ? (w - 1 + 31) / 32 * 32 + 1 : w;
 }
-// byte offset of the flush coefficients (skeleton layout) after `words`
-// 32-bit accumulator words
-RG_HD inline size_t scatter_coef_offset(size_t words) { return (words * 4 + 15) / 16 * 16; }
 
 struct ColFftArgs {       // K2 (forward column FFT) and K4 (inverse column FFT)
     int n1, n2;
@@ -291,10 +299,10 @@ struct ProjArgs {
     const float* frag;    // null: FP32 pass
     int mtiles;           // row blocks of 8 (<= 8)
     int ksteps;           // node steps of 8 in frag (a multiple of 2)
-    // the scatter flush's tensor-core section (ScatterArgs::proj_frag; null
-    // where the grid has none)
-    const float* flush;
-    int flush_ks, flush_nr;
+    // the scatter's flush (ScatterArgs::proj): the coefficients' (hi, lo) parts,
+    // rows in flush_nr blocks of 8, flush_np nodes each (0 blocks: not made)
+    const float2* flush;
+    int flush_nr, flush_np;
 };
 // TF32 (10-bit mantissa) rounding to nearest even, as the host prepares the
 // tensor-core operands; x - tf32(x) is exact in FP32
@@ -405,8 +413,8 @@ RG_HD inline bool fx_wide(int cmax) { return cmax > kFxNarrowMaxLines; }
 
 // --- launchers (rg_kernels.cu) ---------------------------------------------------
 int launch_prepare_lines(const double* v0_d, const double* s_d, int64_t n, double c2_tref,
-                         float2* v0_out, float* ls2_out, int* unsorted_flag, cudaStream_t st);
-int launch_col_index(const float2* v0, int64_t n, double vmin, double dv, int c_min, int count,
+                         float* vh_out, float* vl_out, float* ls2_out, int* unsorted_flag, cudaStream_t st);
+int launch_col_index(const float* vh, const float* vl, int64_t n, double vmin, double dv, int c_min, int count,
                      int64_t* col_start, cudaStream_t st);
 // max over grid columns of the lines within E columns (fixed-point bound), into *cmax
 int launch_col_cmax(const int64_t* col_start, int col_off, int col_count, int n_v, int E, int* cmax,

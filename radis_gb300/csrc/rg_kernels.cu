@@ -36,14 +36,15 @@ __device__ __forceinline__ void two_sum(float a, float b, float& s, float& e) {
 // line preparation at upload: (hi, lo) split of v0 and log2 of the intensity
 // ---------------------------------------------------------------------------
 __global__ void k_prepare_lines(const double* __restrict__ v0, const double* __restrict__ s, int64_t n,
-                                double c2_tref, float2* __restrict__ v0_out, float* __restrict__ ls2,
-                                int* unsorted) {
+                                double c2_tref, float* __restrict__ vh, float* __restrict__ vl,
+                                float* __restrict__ ls2, int* unsorted) {
     int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (i >= n) return;
     double v = v0[i];
     float hi = (float)v;
     float lo = (float)(v - (double)hi);
-    v0_out[i] = make_float2(hi, lo);
+    vh[i] = hi;
+    vl[i] = lo;
     double si = s[i];
     // log2 S_ref - log2(1 - exp(-c2 v0 / Tref)) : the stimulated-emission
     // denominator of base.py:2676 is constant per line
@@ -65,17 +66,21 @@ __device__ __forceinline__ SplitTarget split_target(double t) {
     s.lo = __double2float_ru(t - (double)s.hi);
     return s;
 }
-__device__ __forceinline__ bool below(float2 w, SplitTarget t) { return w.x < t.hi || (w.x == t.hi && w.y < t.lo); }
+struct SplitList {   // a list's positions
+    const float* __restrict__ hi;
+    const float* __restrict__ lo;
+};
+__device__ __forceinline__ bool below(float hi, float lo, SplitTarget t) { return hi < t.hi || (hi == t.hi && lo < t.lo); }
+__device__ __forceinline__ bool below(SplitList v, int64_t i, SplitTarget t) { return below(v.hi[i], v.lo[i], t); }
 
 // First line index with v0 >= target, by one warp: 32 pivots per step, so a list
 // of 10M lines takes 5 dependent loads instead of 24.
-__device__ __forceinline__ int64_t warp_lower_bound(const float2* __restrict__ v0, int64_t n, SplitTarget target,
-                                                    int lane) {
+__device__ __forceinline__ int64_t warp_lower_bound(SplitList v0, int64_t n, SplitTarget target, int lane) {
     int64_t lo = 0, hi = n;   // the answer lies in [lo, hi]
     while (lo < hi) {
         // pivots lo <= p_0 <= ... <= p_31 < hi; v0 ascends, so the lanes below the target come first
         const int64_t p = lo + ((hi - lo) * lane >> 5);
-        const int nb = __popc(__ballot_sync(0xffffffffu, below(v0[p], target)));
+        const int nb = __popc(__ballot_sync(0xffffffffu, below(v0, p, target)));
         const int64_t a = lo + ((hi - lo) * (nb - 1) >> 5), b = lo + ((hi - lo) * nb >> 5);
         if (nb == 0) return lo;
         if (nb < 32) hi = b;
@@ -91,8 +96,8 @@ __device__ __forceinline__ int64_t warp_lower_bound(const float2* __restrict__ v
 // list per column, compared in FP64: 76 us on 5M lines x 400 001 columns, 20 us on
 // 600k lines x 116k columns, alone on a cold GPU; now 25 and 9.)
 constexpr int kColStage = 2048;
-__global__ void __launch_bounds__(256) k_col_index(const float2* __restrict__ v0, int64_t n, double vmin, double dv,
-                                                   int c_min, int count, int64_t* __restrict__ col_start) {
+__global__ void __launch_bounds__(256) k_col_index(SplitList v0, int64_t n, double vmin, double dv, int c_min, int count,
+                                                   int64_t* __restrict__ col_start) {
     __shared__ int64_t ends[2];
     __shared__ float2 part[kColStage];
     const int idx = blockIdx.x * 256 + threadIdx.x;
@@ -108,7 +113,7 @@ __global__ void __launch_bounds__(256) k_col_index(const float2* __restrict__ v0
     const int m = (int)min(ends[1] - first, (int64_t)0x7fffffff);
     const bool staged = m <= kColStage;
     if (staged) {
-        for (int i = threadIdx.x; i < m; i += 256) part[i] = v0[first + i];
+        for (int i = threadIdx.x; i < m; i += 256) part[i] = make_float2(v0.hi[first + i], v0.lo[first + i]);
         __syncthreads();
     }
     if (idx >= count) return;
@@ -118,7 +123,7 @@ __global__ void __launch_bounds__(256) k_col_index(const float2* __restrict__ v0
         int l = 0, h = m;
         while (l < h) {
             const int mid = (l + h) >> 1;
-            if (below(part[mid], target))
+            if (below(part[mid].x, part[mid].y, target))
                 l = mid + 1;
             else
                 h = mid;
@@ -129,13 +134,13 @@ __global__ void __launch_bounds__(256) k_col_index(const float2* __restrict__ v0
             const int64_t span = hi - lo;
             int nb = 0;
 #pragma unroll
-            for (int i = 1; i < 8; ++i) nb += below(v0[lo + (span * i >> 3)], target);
+            for (int i = 1; i < 8; ++i) nb += below(v0, lo + (span * i >> 3), target);
             const int64_t a = lo + (span * nb >> 3), b = lo + (span * (nb + 1) >> 3);
             if (nb < 7) hi = b;   // v0[b] is not below the target
             if (nb > 0)
                 lo = a + 1;          // v0[a] is
             else if (span < 8) {     // the first part may be empty: look at lo itself
-                if (below(v0[lo], target))
+                if (below(v0, lo, target))
                     ++lo;
                 else
                     hi = lo;
@@ -161,10 +166,15 @@ __global__ void k_col_cmax(const int64_t* __restrict__ col_start, int col_off, i
 // ---------------------------------------------------------------------------
 // K1: fused line scaling + LDM scatter into a shared-memory tile
 // ---------------------------------------------------------------------------
-// Tile layout [node][pitch], pitch 1 (mod 32): column c of node n lies in
-// bank (n + c) mod 32.  The lanes of a warp hold neighbouring (sorted) lines,
-// i.e. the same few columns at scattered nodes, so their atomics spread over
-// the banks, and every address is a row base plus a column offset.
+// A tile holds only the node rows that its lines can reach.  The Gaussian
+// width is proportional to v0, so the lines of a few hundred columns lie
+// between two neighbouring Gaussian nodes, or around one: two or three of the
+// grid's Gaussian rows times all Lorentzian ones, from row l_base on.  (Tiles
+// of every node: 128 rows instead of 32-48 on the 8 x 16 grid, 288 instead of
+// 48-72 on 12 x 24; with them went 3-4 times the flush work and, on the larger
+// grid, 1.7 GB of zeros written and read back per spectrum.)  Row pitch 4 (mod
+// 32) words: the flush's fragment loads (4 nodes two apart x 8 columns) touch
+// 32 banks, and the nodes of one column eight.
 
 // --- TMA (cp.async.bulk) + mbarrier helpers ---------------------------------
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -200,34 +210,14 @@ __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
 }
 // Bounded wait (`limit` SM clock cycles); false when it gives up.
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, long long limit = kScatWaitCycles) {
+    if (mbar_try_wait(bar, parity)) return true;
     const long long t0 = clock64();
-    while (!mbar_try_wait(bar, parity))
+    for (;;) {   // the clock every 16 tries: the waiting warps share the issue slots
+#pragma unroll 1
+        for (int i = 0; i < 16; ++i)
+            if (mbar_try_wait(bar, parity)) return true;
         if (clock64() - t0 > limit) return false;
-    return true;
-}
-
-struct Stage {
-    const float2* v0;
-    const float* ls2;
-    const float* el;
-    const float* ga;
-    const float* gs;
-    const float* na;
-    const float* dl;
-    const uint8_t* iso;
-};
-
-__device__ __forceinline__ Stage stage_view(unsigned char* base, int chunk, bool has_dl, bool has_iso) {
-    Stage s;
-    s.v0 = reinterpret_cast<const float2*>(base);
-    s.ls2 = reinterpret_cast<const float*>(base + 8 * chunk);
-    s.el = reinterpret_cast<const float*>(base + 12 * chunk);
-    s.ga = reinterpret_cast<const float*>(base + 16 * chunk);
-    s.gs = reinterpret_cast<const float*>(base + 20 * chunk);
-    s.na = reinterpret_cast<const float*>(base + 24 * chunk);
-    s.dl = has_dl ? reinterpret_cast<const float*>(base + 28 * chunk) : nullptr;
-    s.iso = has_iso ? reinterpret_cast<const uint8_t*>(base + 32 * chunk) : nullptr;
-    return s;
+    }
 }
 
 // One thread: copy lines [start, start + count) of every column into a stage
@@ -236,20 +226,18 @@ __device__ __forceinline__ void issue_chunk(const ScatterArgs& a, unsigned char*
                                             int count) {
     const uint32_t cp = (uint32_t)((count + kLinePad - 1) / kLinePad * kLinePad);
     const int ch = a.chunk;
-    uint32_t bytes = cp * 8 + cp * 4 * 5;
-    if (a.dl) bytes += cp * 4;
-    if (a.iso) bytes += cp;
     // the buffer was last read through the generic proxy
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    mbar_expect_tx(bar, bytes);
-    tma_load_1d(base, a.v0 + start, cp * 8, bar);
+    mbar_expect_tx(bar, cp * (28 + (a.dl ? 4 : 0) + (a.iso ? 1 : 0)));
+    tma_load_1d(base, a.vh + start, cp * 4, bar);
+    tma_load_1d(base + 4 * ch, a.vl + start, cp * 4, bar);
     tma_load_1d(base + 8 * ch, a.ls2 + start, cp * 4, bar);
     tma_load_1d(base + 12 * ch, a.el + start, cp * 4, bar);
     tma_load_1d(base + 16 * ch, a.ga + start, cp * 4, bar);
     tma_load_1d(base + 20 * ch, a.gs + start, cp * 4, bar);
     tma_load_1d(base + 24 * ch, a.na + start, cp * 4, bar);
     if (a.dl) tma_load_1d(base + 28 * ch, a.dl + start, cp * 4, bar);
-    if (a.iso) tma_load_1d(base + 32 * ch, a.iso + start, cp, bar);
+    if (a.iso) tma_load_1d(base + (a.dl ? 32 : 28) * ch, a.iso + start, cp, bar);
 }
 
 // TF32 operands (round to nearest, ties away) and mma.sync m16n8k8 with FP32
@@ -323,188 +311,304 @@ __device__ __forceinline__ float line_intensity(const ScatterArgs& a, float v0, 
 template <bool W> struct Fx;
 template <> struct Fx<false> {
     static constexpr int kWidth = 31;
-    __device__ static void add(unsigned* t, int, float v) { atomicAdd(t, __float2uint_rn(v)); }
+    // the 8 cells of a line: columns c and c + 1 of rows 0, 1, dg, dg + 1 (in pitches)
+    __device__ static void add8(unsigned* t, int pitch, int dg, int, const float (&a)[4], const float (&b)[4]) {
+        unsigned* row[4] = {t, t + pitch, t + dg, t + dg + pitch};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            atomicAdd(row[i], __float2uint_rn(a[i]));
+            atomicAdd(row[i] + 1, __float2uint_rn(b[i]));
+        }
+    }
     __device__ static float value(const unsigned* t, int) { return __uint2float_rn(*t); }
 };
 template <> struct Fx<true> {
     static constexpr int kWidth = 63;
-    __device__ static void add(unsigned* t, int hi_off, float v) {
-        const unsigned long long u = __float2ull_rn(v);
-        const unsigned lo = (unsigned)u;
-        const unsigned old = atomicAdd(t, lo);
-        const unsigned hi = (unsigned)(u >> 32) + (old + lo < old ? 1u : 0u);
-        if (hi) atomicAdd(t + hi_off, hi);
+    // all low words first: the old values come back while the next adds go out
+    __device__ static void add8(unsigned* t, int pitch, int dg, int hi_off, const float (&a)[4], const float (&b)[4]) {
+        unsigned* row[4] = {t, t + pitch, t + dg, t + dg + pitch};
+        unsigned hi[8], lo[8], old[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const unsigned long long u = __float2ull_rn(i & 1 ? b[i >> 1] : a[i >> 1]);
+            lo[i] = (unsigned)u;
+            hi[i] = (unsigned)(u >> 32);
+            old[i] = atomicAdd(row[i >> 1] + (i & 1), lo[i]);
+        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            hi[i] += old[i] + lo[i] < lo[i] ? 1u : 0u;
+            if (hi[i]) atomicAdd(row[i >> 1] + (i & 1) + hi_off, hi[i]);
+        }
     }
     __device__ static float value(const unsigned* t, int hi_off) {
         return __ull2float_rn(((unsigned long long)t[hi_off] << 32) | *t);
     }
 };
 
-// Scale + scatter of the lines of one staged chunk into the tile accumulator
-// (`tile`: this lane's copy).
+// --- the same on two lines per thread ----------------------------------------
+// Packed FP32 (fadd2 / ffma2): a pair of lines costs the issue slots of one.
+__device__ __forceinline__ float2 neg2(float2 a) { return make_float2(-a.x, -a.y); }
+__device__ __forceinline__ float2 dup2(float x) { return make_float2(x, x); }
+__device__ __forceinline__ float2 sub2(float2 a, float2 b) { return __fadd2_rn(a, neg2(b)); }
+__device__ __forceinline__ void two_sum2(float2 a, float2 b, float2& s, float2& e) {
+    s = __fadd2_rn(a, b);
+    const float2 bb = sub2(s, a);
+    e = __fadd2_rn(sub2(a, sub2(s, bb)), sub2(b, bb));
+}
+// floor for |x| < 2^22: 1.5 2^23 + x rounded down has ulp 1.  From 2^22 to
+// 2^24 the result is the even number below (a position's fraction is floored
+// once more); values beyond stay out of every window.
+__device__ __forceinline__ float2 floor2(float2 x) {
+    const float m = 12582912.f;
+    return __fadd2_rn(__fadd2_rd(x, dup2(m)), dup2(-m));
+}
+__device__ __forceinline__ float2 clamp2(float2 x, float lo, float hi) {
+    return make_float2(fminf(fmaxf(x.x, lo), hi), fminf(fmaxf(x.y, lo), hi));
+}
+
+// What a tile's lines need of it.
+struct TileView {
+    float k_start, k_lo, k_hi;   // first column; positions whose line touches the tile's columns
+    float l_lo, l_hi;            // Gaussian cells (l0) of its lines
+    int l_base, l_rows;          // first Gaussian row, rows in use
+};
+__device__ __forceinline__ TileView tile_view(const ScatterArgs& a, int tile) {
+    TileView t;
+    const int k0 = tile * a.TK, tk = min(a.TK, a.n_v - k0);
+    t.k_start = (float)k0;
+    t.k_lo = (float)max(k0 - 1, 0);
+    t.k_hi = (float)min(k0 + tk - 1, a.n_v - 2);   // dropped beyond (cmdFillLDM.comp:102)
+    // Gaussian coordinates of the first and last line position, with room for rounding
+    const float va = fmaxf(fmaf((float)(k0 - 1 - a.margin_cols), a.v_step, a.v_lo), a.v_bot);
+    const float vb = fmaxf(fmaf((float)(k0 + tk + a.margin_cols), a.v_step, a.v_lo), a.v_bot);
+    const float pa = fmaf(lg2(va * a.inv_vref), a.lgG_scale, a.cG_lo) - 0.05f;
+    const float pb = fmaf(lg2(vb * a.inv_vref), a.lgG_scale, a.cG_hi) + 0.05f;
+    const float lb = fminf(fmaxf(floorf(pa), 0.f), (float)(a.NG - a.win));
+    const float le = fminf(fmaxf(floorf(pb), lb), lb + (float)(a.win - 2));
+    t.l_lo = lb;
+    t.l_hi = le;
+    t.l_base = (int)lb;
+    t.l_rows = (int)(le - lb) + 2;
+    return t;
+}
+
+// Lines 2p and 2p + 1 of a staged chunk (`two`: the second exists) into the
+// tile accumulator (`tile`: this lane's copy).  A line one column left of the
+// tile or on its last column also adds to a word beyond that column: padding
+// that nothing reads.  Returns the lines that count as the tile's.
 template <bool W>
-__device__ __forceinline__ unsigned scatter_chunk(const ScatterArgs& a, const Stage& st, int count, int k_start,
-                                                  int tk, unsigned* tile, float fxs, int t0, int nt) {
-    unsigned counted = 0;
-    const int hi_off = a.n_nodes * a.pitch;
-    for (int j = t0; j < count; j += nt) {
-        const float2 v = st.v0[j];
-        const float dl = st.dl ? st.dl[j] : 0.f;
-        float fk, tv;
-        line_position(a, v, dl, fk, tv);
-        if (!(fk >= 0.f) || fk + 1.f >= (float)a.n_v) continue;   // drop (cmdFillLDM.comp:102)
-        const int k0 = (int)fk;
-        const int c0 = k0 - k_start;
-        const bool own0 = (unsigned)c0 < (unsigned)tk;
-        const bool own1 = (unsigned)(c0 + 1) < (unsigned)tk;
-        if (!(own0 || own1)) continue;
-        if (own0) ++counted;
-        const int is = st.iso ? (int)st.iso[j] : 0;
-        int l0, m0;
-        float tG, tL;
-        line_nodes(a, v.x, st.ga[j], st.gs[j], st.na[j], is, l0, m0, tG, tL);
-        const float I = line_intensity(a, v.x, st.el[j], st.ls2[j], is) * fxs;
-        const float I1 = tv * I;
-        const float I0 = I - I1;
-        const float w11 = tG * tL;
-        const float w10 = tG - w11;          // tG (1 - tL)
-        const float w01 = tL - w11;          // (1 - tG) tL
-        const float w00 = 1.f - tG - w01;    // (1 - tG)(1 - tL)
-        const int pitch = a.pitch;
-        const int dL = a.NL * pitch;                          // next wG node
-        unsigned* t = tile + (l0 * a.NL + m0) * pitch + c0;   // (l0, m0) at column c0
-        if (own0) {
-            Fx<W>::add(t, hi_off, I0 * w00);
-            Fx<W>::add(t + pitch, hi_off, I0 * w01);
-            Fx<W>::add(t + dL, hi_off, I0 * w10);
-            Fx<W>::add(t + dL + pitch, hi_off, I0 * w11);
+__device__ __forceinline__ unsigned scatter_pair(const ScatterArgs& a, const TileView& tv, const unsigned char* st, int p,
+                                                 bool two, unsigned* tile, float fxs) {
+    const LinePairs& k = a.k2;
+    const int ch4 = 4 * a.chunk;
+    const unsigned char* q = st + 8 * p;
+    auto col = [&](int i) { return *reinterpret_cast<const float2*>(q + i * ch4); };
+    const float2 vh = col(0);
+    // position (line_position)
+    float2 s, e;
+    two_sum2(vh, k.neg_vmin_hi, s, e);
+    float2 t = sub2(col(1), k.vmin_lo);
+    if (a.dl) t = __ffma2_rn(col(7), k.p_atm, t);
+    e = __fadd2_rn(e, t);
+    const float2 pos = __fmul2_rn(s, k.inv_dv_hi);
+    const float2 pe = __fadd2_rn(__ffma2_rn(s, k.inv_dv_hi, neg2(pos)), __ffma2_rn(s, k.inv_dv_lo, __fmul2_rn(e, k.inv_dv_hi)));
+    float2 fk = floor2(pos);
+    float2 f = __fadd2_rn(sub2(pos, fk), pe);
+    const float2 fl = floor2(f);
+    fk = __fadd2_rn(fk, fl);
+    f = sub2(f, fl);
+    const bool ok0 = fk.x >= tv.k_lo && fk.x <= tv.k_hi;
+    const bool ok1 = two && fk.y >= tv.k_lo && fk.y <= tv.k_hi;
+    if (!(ok0 || ok1)) return 0;
+    // nodes (line_nodes)
+    float2 cG = k.cG, bh = k.bI_hi, bl = k.bI_lo;
+    if (a.iso) {
+        const unsigned char* is = st + (a.dl ? 8 : 7) * ch4 + 2 * p;
+        const int i0 = is[0], i1 = two ? is[1] : i0;
+        cG = make_float2(a.cG[i0], a.cG[i1]);
+        bh = make_float2(a.bI_hi[i0], a.bI_hi[i1]);
+        bl = make_float2(a.bI_lo[i0], a.bI_lo[i1]);
+    }
+    const float2 xv = __fmul2_rn(vh, k.inv_vref);
+    const float2 pl = __ffma2_rn(make_float2(lg2(xv.x), lg2(xv.y)), k.lgG_scale, cG);
+    const float2 ga = col(4);
+    const float2 gam = __ffma2_rn(k.x_self, sub2(col(5), ga), ga);
+    const float2 pm = __ffma2_rn(make_float2(lg2(gam.x), lg2(gam.y)), k.lgL_scale, __ffma2_rn(col(6), k.tL, k.cL));
+    const float2 l0 = clamp2(floor2(pl), tv.l_lo, tv.l_hi);
+    const float2 m0 = clamp2(floor2(pm), 0.f, (float)(a.NL - 2));
+    const float2 tG = sub2(pl, l0), tL = sub2(pm, m0);
+    const float2 row = __ffma2_rn(sub2(l0, dup2(tv.l_lo)), k.n_l, m0);
+    const float2 at = __ffma2_rn(row, dup2((float)a.pitch), sub2(fk, dup2(tv.k_start)));
+    // intensity (line_intensity), in accumulator units
+    const float2 el = col(3);
+    const float2 ph = __fmul2_rn(el, k.aT_hi);
+    const float2 pe2 = __ffma2_rn(el, k.aT_lo, __ffma2_rn(el, k.aT_hi, neg2(ph)));
+    float2 s1, f1, s2, f2;
+    two_sum2(ph, bh, s1, f1);
+    two_sum2(s1, col(2), s2, f2);
+    const float2 arg = __fadd2_rn(s2, __fadd2_rn(__fadd2_rn(__fadd2_rn(f1, f2), pe2), bl));
+    const float2 xs = __fmul2_rn(vh, k.stim);
+    const float2 em = sub2(dup2(1.f), make_float2(ex2(-xs.x), ex2(-xs.y)));
+    const float2 I = __fmul2_rn(__fmul2_rn(make_float2(ex2(arg.x), ex2(arg.y)), em), dup2(fxs));
+    // weights
+    const float2 I1 = __fmul2_rn(f, I), I0 = sub2(I, I1);
+    const float2 w11 = __fmul2_rn(tG, tL);
+    const float2 w10 = sub2(tG, w11);                  // tG (1 - tL)
+    const float2 w01 = sub2(tL, w11);                  // (1 - tG) tL
+    const float2 w00 = sub2(sub2(dup2(1.f), tG), w01);   // (1 - tG)(1 - tL)
+    const float2 a00 = __fmul2_rn(I0, w00), a01 = __fmul2_rn(I0, w01), a10 = __fmul2_rn(I0, w10), a11 = __fmul2_rn(I0, w11);
+    const float2 b00 = __fmul2_rn(I1, w00), b01 = __fmul2_rn(I1, w01), b10 = __fmul2_rn(I1, w10), b11 = __fmul2_rn(I1, w11);
+    const int pitch = a.pitch, dG = a.NL * pitch, hi_off = a.rows * pitch;
+    if (ok0) {
+        const float x0[4] = {a00.x, a01.x, a10.x, a11.x}, x1[4] = {b00.x, b01.x, b10.x, b11.x};
+        Fx<W>::add8(tile + __float2int_rn(at.x), pitch, dG, hi_off, x0, x1);
+    }
+    if (ok1) {
+        const float x0[4] = {a00.y, a01.y, a10.y, a11.y}, x1[4] = {b00.y, b01.y, b10.y, b11.y};
+        Fx<W>::add8(tile + __float2int_rn(at.y), pitch, dG, hi_off, x0, x1);
+    }
+    return a.in_window ? (ok0 && fk.x >= tv.k_start) + (ok1 && fk.y >= tv.k_start) : 0u;
+}
+
+// Columns [c, c + NC) of a finished tile, by one warp.
+// Sum of the tile's copies into the first (integer sums: exact), the others zeroed.
+template <bool W, int NC>
+__device__ __forceinline__ void fold_copies(const ScatterArgs& a, unsigned* tile, int c, int rows, int lane) {
+    const int hi_off = a.rows * a.pitch;
+    for (int i = lane; i < rows * NC; i += 32) {
+        unsigned* w = tile + (i / NC) * a.pitch + c + i % NC;
+        unsigned long long s = 0;
+        for (int q = 0; q < a.copies; ++q, w += a.copy_words) {
+            s += W ? ((unsigned long long)w[hi_off] << 32) | w[0] : w[0];
+            w[0] = 0;
+            if (W) w[hi_off] = 0;
         }
-        if (own1) {
-            Fx<W>::add(t + 1, hi_off, I1 * w00);
-            Fx<W>::add(t + 1 + pitch, hi_off, I1 * w01);
-            Fx<W>::add(t + 1 + dL, hi_off, I1 * w10);
-            Fx<W>::add(t + 1 + dL + pitch, hi_off, I1 * w11);
+        w -= a.copies * a.copy_words;
+        w[0] = (unsigned)s;
+        if (W) w[hi_off] = (unsigned)(s >> 32);
+    }
+    __syncwarp();
+}
+template <bool W, int NC>
+__device__ __forceinline__ void zero_columns(const ScatterArgs& a, unsigned* tile, int c, int rows, int lane) {
+    __syncwarp();
+    for (int i = lane; i < rows * (NC / 4); i += 32) {
+        unsigned* w = tile + (i / (NC / 4)) * a.pitch + c + 4 * (i % (NC / 4));
+        *reinterpret_cast<uint4*>(w) = make_uint4(0u, 0u, 0u, 0u);
+        if (W) *reinterpret_cast<uint4*>(w + a.rows * a.pitch) = make_uint4(0u, 0u, 0u, 0u);
+        else if (a.copies == 2) {   // (the second copy is not 16-byte aligned)
+            w += a.copy_words;
+            w[0] = w[1] = w[2] = w[3] = 0u;
         }
     }
-    return counted;
 }
 
-// Zero `words` accumulator words from thread `i0` in steps of `step` threads,
-// 16 bytes per store (the tile starts on a 16-byte boundary).
-__device__ __forceinline__ void zero_tile(unsigned* tile, int words, int i0, int step) {
-    const int n16 = words >> 2;
-    uint4* z = reinterpret_cast<uint4*>(tile);
-    for (int i = i0; i < n16; i += step) z[i] = make_uint4(0u, 0u, 0u, 0u);
-    for (int i = (n16 << 2) + i0; i < words; i += step) tile[i] = 0;
+// Coefficients of eight nodes from `node` on, rows 8 nr .. 8 nr + 7, as one
+// lane's B fragment (the window's padding rows hold zeros: any coefficient does).
+__device__ __forceinline__ float4 proj_frag(const ScatterArgs& a, int nr, int node, int lane) {
+    const float2* p = a.proj + ((nr * a.proj_np + min(node + 2 * (lane & 3), a.proj_np - 2)) << 3) + (lane >> 2);
+    const float2 u = __ldg(p), v = __ldg(p + 8);
+    return make_float4(u.x, u.y, v.x, v.y);
 }
 
-// Sum the tile's copies into the first one (integer sums: exact).
-template <bool W>
-__device__ __forceinline__ void fold_copies(const ScatterArgs& a, unsigned* tile, int i0, int step) {
-    const int n = a.n_nodes * a.pitch;
-    for (int i = i0; i < n; i += step) {
-        if constexpr (W) {
-            unsigned long long s = 0;
-            for (int c = 0; c < a.copies; ++c) {
-                const unsigned* t = tile + c * a.copy_words + i;
-                s += ((unsigned long long)t[n] << 32) | t[0];
-            }
-            tile[i] = (unsigned)s;
-            tile[n + i] = (unsigned)(s >> 32);
-        } else {
-            unsigned s = 0;
-            for (int c = 0; c < a.copies; ++c) s += tile[c * a.copy_words + i];
-            tile[i] = s;
-        }
-    }
-}
-
-// Skeleton rows of a finished 32-bit tile on the tensor cores: Y^T[columns x
-// rows] = T^T[columns x nodes] C^T[nodes x rows] with mma.sync m16n8k8 TF32,
-// each product split into three (hi hi + lo hi + hi lo; x = hi + lo, hi =
-// tf32(x), lo = tf32(x - hi)).  Warp task: 16 columns (M) x the NR row blocks
-// of 8 (N); nodes (K) eight per step in the order of the staged node table
-// offs[s][t] = (node(s, t), node(s, t + 4)) x pitch.  Tile rows have a pitch
-// of 1 (mod 32) words and the table puts the nodes of t = 0..3 in the bank
-// classes v, v + 8, v + 16, v + 24, so the A loads (column g / g + 8, node t /
-// t + 4) are conflict-free; frag[s][nr][lane] = the coefficients' B fragments
-// (b0, b1 hi, then lo), zero where the table repeats a node.
-template <int NR, int U>
-__device__ __forceinline__ void flush_tc(const ScatterArgs& a, const unsigned* tile, const float4* frag,
-                                         const int2* offs, int k_start, int tk, float inv_fx, int cw, int ncw,
-                                         int lane) {
+// Skeleton rows of 16 columns on the tensor cores: Y^T[columns x rows] =
+// T^T[columns x nodes] C^T[nodes x rows] with mma.sync m16n8k8 TF32, each
+// product split into three (hi hi + lo hi + hi lo; x = hi + lo, hi = tf32(x),
+// lo = tf32(x - hi)): columns as M, the NR row blocks of 8 as N, the tile's
+// nodes as K, eight per step (past the rows in use the tile holds zeros); k =
+// t, t + 4 are nodes 2 t, 2 t + 1 of a step, 8 banks apart.  Two sums per
+// output keep the chains of dependent MMAs short.  frag: the coefficients of
+// the tile's nodes as B fragments, [step][row block][lane] (node 2 t hi, lo,
+// node 2 t + 1 hi, lo), in shared memory (through L1 the reads missed: a
+// third of the 5M-line scatter's time), where it has the room (kFrags).
+template <bool W, int NR, bool kFrags>
+__device__ __forceinline__ void project_columns(const ScatterArgs& a, int steps, int first, const unsigned* tile,
+                                                const float4* frag, int c, int nr0, int k_start, int tk, float inv_fx,
+                                                int lane) {
     const int g = lane >> 2, t = lane & 3;
-    const int n_mt = (tk + 15) >> 4;
-    for (int mt = cw; mt < n_mt; mt += ncw) {
-        const unsigned* col = tile + (mt << 4) + g;
-        float d[NR][4];
+    const int hi_off = a.rows * a.pitch;
+    const bool two = !W && a.copies == 2;   // two copies are added up here, more by fold_copies
+    const unsigned* col = tile + 2 * t * a.pitch + c + g;
+    const float4* cf = frag + nr0 * 32 + lane;
+    float d[NR][4], e[NR][4];
 #pragma unroll
-        for (int nr = 0; nr < NR; ++nr)
+    for (int nr = 0; nr < NR; ++nr)
 #pragma unroll
-            for (int i = 0; i < 4; ++i) d[nr][i] = 0.f;
-#pragma unroll U
-        for (int s = 0; s < a.proj_ks; ++s) {
-            const int2 o = offs[s * 4 + t];
-            const float v[4] = {__uint2float_rn(col[o.x]), __uint2float_rn(col[o.x + 8]),
-                                __uint2float_rn(col[o.y]), __uint2float_rn(col[o.y + 8])};
-            uint32_t ah[4], al[4];
+        for (int i = 0; i < 4; ++i) d[nr][i] = e[nr][i] = 0.f;
+#pragma unroll 2
+    for (int s = 0; s < steps; ++s, col += 8 * a.pitch, cf += 32 * a.proj_nr) {
+        float4 b[NR];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                ah[i] = tf32_rna(v[i]);
-                al[i] = tf32_rna(v[i] - __uint_as_float(ah[i]));
-            }
-            float4 f[NR];
+        for (int nr = 0; nr < NR; ++nr) b[nr] = kFrags ? cf[nr * 32] : proj_frag(a, nr0 + nr, first + 8 * s, lane);
+        const unsigned* p[4] = {col, col + 8, col + a.pitch, col + a.pitch + 8};
+        uint32_t ah[4], al[4];
 #pragma unroll
-            for (int nr = 0; nr < NR; ++nr) f[nr] = frag[(s * NR + nr) * 32 + lane];
-#pragma unroll
-            for (int nr = 0; nr < NR; ++nr) mma_tf32(d[nr], ah, __float_as_uint(f[nr].x), __float_as_uint(f[nr].y));
-#pragma unroll
-            for (int nr = 0; nr < NR; ++nr) mma_tf32(d[nr], al, __float_as_uint(f[nr].x), __float_as_uint(f[nr].y));
-#pragma unroll
-            for (int nr = 0; nr < NR; ++nr) mma_tf32(d[nr], ah, __float_as_uint(f[nr].z), __float_as_uint(f[nr].w));
+        for (int i = 0; i < 4; ++i) {
+            float v;
+            if constexpr (W) v = Fx<W>::value(p[i], hi_off);
+            else v = __uint2float_rn(two ? p[i][0] + p[i][a.copy_words] : p[i][0]);
+            ah[i] = tf32_rna(v);
+            al[i] = tf32_rna(v - __uint_as_float(ah[i]));
         }
-        // d[nr][i]: column 16 mt + g + 8 (i / 2), row 8 nr + 2 t + i % 2
-        const int c = (mt << 4) + g;
 #pragma unroll
-        for (int nr = 0; nr < NR; ++nr)
+        for (int nr = 0; nr < NR; ++nr) mma_tf32(e[nr], al, __float_as_uint(b[nr].x), __float_as_uint(b[nr].z));
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const int r = 8 * nr + 2 * t + (i & 1);
-                const int cc = c + 8 * (i >> 1);
-                if (r < a.proj_rows && cc < tk) __stcs(a.ldm + (int64_t)r * a.row_stride + k_start + cc, d[nr][i] * inv_fx);
-            }
+        for (int nr = 0; nr < NR; ++nr) mma_tf32(d[nr], ah, __float_as_uint(b[nr].x), __float_as_uint(b[nr].z));
+#pragma unroll
+        for (int nr = 0; nr < NR; ++nr) mma_tf32(e[nr], ah, __float_as_uint(b[nr].y), __float_as_uint(b[nr].w));
     }
+    // d[nr][i]: column c + g + 8 (i / 2), row 8 (nr0 + nr) + 2 t + i % 2
+#pragma unroll
+    for (int nr = 0; nr < NR; ++nr)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int r = 8 * (nr0 + nr) + 2 * t + (i & 1);
+            const int cc = c + g + 8 * (i >> 1);
+            if (r < a.proj_rows && cc < tk)
+                __stcs(a.ldm + (int64_t)r * a.row_stride + k_start + cc, (d[nr][i] + e[nr][i]) * inv_fx);
+        }
 }
-
-// Persistent, warp-specialised scatter: CTA b owns tiles b, b + G, b + 2G,
-// ...  Warp 0 (one thread) is the producer: it streams the tiles' line
-// records chunk by chunk into a ring of `stages` buffers with TMA bulk copies,
-// each buffer guarded by a "full" mbarrier (TMA completion) and an "empty"
-// one (one arrival per consumer warp).  Warps 1..31 consume: each waits for a
-// chunk, scatters its share of the lines into the tile accumulator (32-bit
-// fixed point, native integer shared atomics, deterministic) and releases the
-// buffer; warps meet only at tile boundaries (a named barrier of the consumer
-// warps) to flush the finished tile to HBM with plain stores.  Every wait is
-// bounded; a wait that gives up sets the error flag and the CTA stops after
-// the copies it issued have landed (bounded).  W: 64-bit sums.  U: unrolling of the tensor-core flush's node
-// steps (4 where registers allow, 1 in the kernel that holds both variants).
-template <bool W, int U = 4>
+// Persistent, warp-specialised scatter: CTA b owns tiles b, b + G, b + 2G, ...
+//  * warp 0 (one thread): streams the tiles' line records chunk by chunk into a
+//    ring of buffers with TMA bulk copies, each buffer guarded by a "full"
+//    mbarrier (TMA completion) and an "empty" one (one arrival per line warp);
+//  * line warps: two lines per lane and chunk, scattered into the tile (fixed
+//    point, native integer shared atomics, deterministic).  The lanes of a
+//    warp take pairs `stride` (odd) apart, so that they lie in different
+//    columns and their adds in different banks;
+//  * flush warps: project (or copy) a finished tile's columns to HBM and zero
+//    them, 16 (32) columns a warp at a time, while the line warps fill the other
+//    of two tile slots ("tfull": one arrival per line warp, "tfree": one per
+//    flush warp; "fmeet": the flush warps around a change of the coefficients
+//    they share).
+// Every wait is bounded; a wait that gives up sets the error flag and its warp
+// stops, the others' waits run out in turn, and the producer stays until the
+// copies it issued have landed (bounded).  W: 64-bit sums.
+// A tile holds the `win` Gaussian rows that its lines can reach, not all of the
+// grid's: 12 x 24 nodes need 72 of 288 rows, so that two tiles of hundreds of
+// columns fit and the flush reads a quarter.  One kernel projects every grid:
+// the node rows never reach memory.  Against one tile of all rows filled and
+// flushed in turn: 5M lines x 400k points 94 -> 57 us (28 bytes a line are 21
+// us of HBM; the shared atomics' wavefronts, the flush's MMA chains and its
+// last tile are the rest), 100M x 1.5M points 1130 + 407 (a projection pass) ->
+// 800 us (HBM: 414 us).  Two CTAs per SM of half the size: 58.6 and 957 us.
+template <bool W>
 __device__ __forceinline__ void scatter_body(const ScatterArgs& a) {
     extern __shared__ __align__(128) unsigned char smem[];
-    const int ch = a.chunk;
-    const int S = a.stages;
-    const size_t sb = scatter_stage_bytes(ch);
+    const int ch = a.chunk, S = a.stages, sb = a.stage_bytes;
     uint64_t* full = reinterpret_cast<uint64_t*>(smem + S * sb);
     uint64_t* empty = full + kScatMaxStages;
-    int2* rng = reinterpret_cast<int2*>(smem + S * sb + 16 * kScatMaxStages);
-    unsigned* tile = reinterpret_cast<unsigned*>(smem + scatter_fixed_smem(ch, S, a.rng_cap));
-    const int pitch = a.pitch;
-    const int hi_off = a.n_nodes * pitch;
+    uint64_t* tfull = empty + kScatMaxStages;
+    uint64_t* tfree = tfull + 2;
+    uint64_t* fmeet = tfree + 2;
+    int2* rng = reinterpret_cast<int2*>(smem + S * sb + 192);
+    unsigned* tiles = reinterpret_cast<unsigned*>(smem + scatter_fixed_smem(sb, S, a.rng_cap));
+    const int slot_words = (a.copies * a.copy_words + 3) & ~3;
     const int G = gridDim.x;
     const int nq = (a.n_tiles - (int)blockIdx.x + G - 1) / G;   // tiles of this CTA (<= a.rng_cap)
-    const int n_words = a.copies * a.copy_words;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int n_cons_warps = (blockDim.x >> 5) - 1;
+    const int lw = a.line_warps, fw = (int)(blockDim.x >> 5) - 1 - lw;
 
     if (nq > a.rng_cap) {   // the host sizes the table for every CTA: never taken
         if (threadIdx.x == 0) atomicExch(a.err, 1u);
@@ -518,31 +622,20 @@ __device__ __forceinline__ void scatter_body(const ScatterArgs& a) {
         const int hi = (int)a.col_start[col_idx(k_start + tk + a.margin_cols)];
         rng[q] = make_int2(lo / kLinePad * kLinePad, hi);   // 16-line aligned start
     }
-    zero_tile(tile, n_words, (int)threadIdx.x, (int)blockDim.x);
-    // skeleton layout: the projection coefficients after the tile, as FP32
-    // [node][row] or (32-bit tiles) the tensor-core flush's B fragments and
-    // node table
-    float* coef = reinterpret_cast<float*>(reinterpret_cast<unsigned char*>(tile) +
-                                           scatter_coef_offset(n_words));
-    const bool proj = a.proj_coef != nullptr;
-    const bool proj_tc = !W && proj && a.proj_frag != nullptr;
-    const int n_frag = proj_tc ? a.proj_ks * a.proj_nr * 32 : 0;
-    const float4* frag_s = reinterpret_cast<const float4*>(coef);
-    const int2* offs_s = reinterpret_cast<const int2*>(frag_s + n_frag);
-    if (proj_tc) {
-        const float4* src = reinterpret_cast<const float4*>(a.proj_frag);
-        for (int i = threadIdx.x; i < n_frag; i += blockDim.x) reinterpret_cast<float4*>(coef)[i] = __ldg(&src[i]);
-        const int* tbl = reinterpret_cast<const int*>(src + n_frag);
-        int* offs = reinterpret_cast<int*>(reinterpret_cast<float4*>(coef) + n_frag);
-        for (int i = threadIdx.x; i < a.proj_ks * 8; i += blockDim.x) offs[i] = __ldg(&tbl[i]) * pitch;
-    } else if (proj) {
-        for (int i = threadIdx.x; i < a.n_real * a.proj_rp; i += blockDim.x) coef[i] = __ldg(&a.proj_coef[i]);
+    {
+        uint4* z = reinterpret_cast<uint4*>(tiles - 4);   // with the words before the first tile
+        for (int i = threadIdx.x; i <= a.slots * slot_words / 4; i += blockDim.x) z[i] = make_uint4(0u, 0u, 0u, 0u);
     }
     if (threadIdx.x == 0) {
         for (int b = 0; b < S; ++b) {
             mbar_init(&full[b], 1);
-            mbar_init(&empty[b], n_cons_warps);
+            mbar_init(&empty[b], lw);
         }
+        for (int b = 0; b < 2; ++b) {
+            mbar_init(&tfull[b], lw);
+            mbar_init(&tfree[b], fw);
+        }
+        mbar_init(fmeet, fw);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
@@ -574,130 +667,123 @@ __device__ __forceinline__ void scatter_body(const ScatterArgs& a) {
         return;
     }
 
-    // consumers
     const float fxs = fx_scale_of(*a.cmax, Fx<W>::kWidth);
-    const float inv_fx = 1.f / fxs;
-    const bool has_dl = a.dl != nullptr, has_iso = a.iso != nullptr;
-    const int ct = threadIdx.x - 32, nct = blockDim.x - 32;
-    const int cw = warp - 1;
-    unsigned* my_tile = tile + (lane & (a.copies - 1)) * a.copy_words;
-    int buf = 0;            // ring slot of the next chunk (chunks consumed mod S)
-    uint32_t par = 0;       // phase parity of its "full" barrier
-    unsigned counted = 0;
-    bool bad = false;
-    for (int q = 0; q < nq; ++q) {
-        const int k_start = ((int)blockIdx.x + q * G) * a.TK;
-        const int tk = min(a.TK, a.n_v - k_start);
-        const int b = rng[q].y;
-        for (int cs = rng[q].x; cs < b && !bad; cs += ch) {
-            // every lane acquires the TMA data through the mbarrier itself
-            const bool ok = mbar_wait(&full[buf], par, a.wait_limit);
-            if (!__all_sync(0xffffffffu, ok)) {
-                bad = true;
-                break;
+    if (warp <= lw) {   // line warps
+        const int w = warp - 1;
+        int buf = 0;            // ring slot of the next chunk (chunks consumed mod S)
+        uint32_t par = 0;       // phase parity of its "full" barrier
+        unsigned counted = 0;
+        for (int q = 0; q < nq; ++q) {
+            const int slot = a.slots == 2 ? q & 1 : 0, use = a.slots == 2 ? q >> 1 : q;
+            const TileView tv = tile_view(a, (int)blockIdx.x + q * G);
+            unsigned* tile = tiles + slot * slot_words + (lane & (a.copies - 1)) * a.copy_words;
+            bool ok = use == 0 || __all_sync(0xffffffffu, mbar_wait(&tfree[slot], (use - 1) & 1, a.wait_limit));
+            const int b = rng[q].y;
+            for (int cs = rng[q].x; cs < b && ok; cs += ch) {
+                // every lane acquires the TMA data through the mbarrier itself
+                ok = __all_sync(0xffffffffu, mbar_wait(&full[buf], par, a.wait_limit));
+                if (!ok) break;
+                const int count = min(ch, b - cs);
+                const int stride = ((count + 63) >> 6) | 1;   // odd, <= lw
+                const int p = lane * stride + w;
+                if (w < stride && 2 * p < count)
+                    counted += scatter_pair<W>(a, tv, smem + buf * sb, p, 2 * p + 1 < count, tile, fxs);
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&empty[buf]);   // this warp is done with the buffer
+                if (++buf == S) {
+                    buf = 0;
+                    par ^= 1u;
+                }
             }
-            counted += scatter_chunk<W>(a, stage_view(smem + buf * sb, ch, has_dl, has_iso), min(ch, b - cs),
-                                        k_start, tk, my_tile, fxs, ct, nct);
+            if (!ok) {   // the same on every lane
+                if (lane == 0) atomicExch(a.err, 1u);
+                return;
+            }
             __syncwarp();
-            if (lane == 0) mbar_arrive(&empty[buf]);   // this warp is done with the buffer
-            if (++buf == S) {
-                buf = 0;
-                par ^= 1u;
-            }
+            if (lane == 0) mbar_arrive(&tfull[slot]);   // this warp is done with the tile
         }
-        // all consumer warps done with the tile (and agree on failures)
-        int any_bad;
-        asm volatile(
-            "{\n .reg .pred p, q;\n setp.ne.u32 p, %1, 0;\n barrier.cta.red.or.pred q, 1, %2, p;\n"
-            " selp.u32 %0, 1, 0, q;\n}\n"
-            : "=r"(any_bad)
-            : "r"((unsigned)bad), "r"(nct)
-            : "memory");
-        if (any_bad) {
-            if (threadIdx.x == 32) atomicExch(a.err, 1u);
+        if (a.in_window) {   // one atomic per warp: per-thread atomics on one word serialise in L2
+            const unsigned tot = __reduce_add_sync(0xffffffffu, counted);
+            if (lane == 0 && tot) atomicAdd(a.in_window, (unsigned long long)tot);
+        }
+        return;
+    }
+
+    // flush warps
+    const float inv_fx = 1.f / fxs;
+    const int w = warp - 1 - lw;
+    float4* frag = reinterpret_cast<float4*>(tiles + a.slots * slot_words);   // of the Gaussian rows from frag_base on
+    int frag_base = -1;
+    uint32_t meet_par = 0;
+    auto meet = [&] {   // the flush warps, bounded as every wait
+        __syncwarp();
+        if (lane == 0) mbar_arrive(fmeet);
+        const bool ok = __all_sync(0xffffffffu, mbar_wait(fmeet, meet_par, a.wait_limit));
+        meet_par ^= 1u;
+        if (!ok && lane == 0) atomicExch(a.err, 1u);
+        return ok;
+    };
+    for (int q = 0; q < nq; ++q) {
+        const int slot = a.slots == 2 ? q & 1 : 0, use = a.slots == 2 ? q >> 1 : q;
+        const int ti = (int)blockIdx.x + q * G;
+        const TileView tv = tile_view(a, ti);
+        const int k_start = ti * a.TK, tk = min(a.TK, a.n_v - k_start);
+        unsigned* tile = tiles + slot * slot_words;
+        const int first = tv.l_base * a.NL;
+        if (a.proj && a.proj_frags && tv.l_base != frag_base) {   // rarely: neighbouring tiles share it
+            frag_base = tv.l_base;
+            if (q && !meet()) return;   // every read of the old ones done
+            for (int i = 32 * w + lane; i < (a.rows >> 3) * a.proj_nr * 32; i += 32 * fw) {
+                const int s = i / (32 * a.proj_nr), nr = (i >> 5) - s * a.proj_nr;
+                frag[i] = proj_frag(a, nr, first + 8 * s, i & 31);
+            }
+            if (!meet()) return;
+        }
+        if (!__all_sync(0xffffffffu, mbar_wait(&tfull[slot], use & 1, a.wait_limit))) {
+            if (lane == 0) atomicExch(a.err, 1u);
             return;
         }
-        if (a.copies > 1) {
-            fold_copies<W>(a, tile, ct, nct);
-            asm volatile("bar.sync 1, %0;" ::"r"(nct) : "memory");
-        }
-        if (proj_tc) {
-            if constexpr (!W) {
-                if (a.proj_nr == 2)
-                    flush_tc<2, U>(a, tile, frag_s, offs_s, k_start, tk, inv_fx, cw, n_cons_warps, lane);
-                else
-                    flush_tc<1, U>(a, tile, frag_s, offs_s, k_start, tk, inv_fx, cw, n_cons_warps, lane);
-            }
-            asm volatile("bar.sync 1, %0;" ::"r"(nct) : "memory");   // every read of the tile done
-            zero_tile(tile, n_words, ct, nct);
-        } else if (proj) {
-            // skeleton rows of the finished tile: warp task (64-column group,
-            // block of 4 rows); lane l sums columns l and l + 32 of its group
-            // (each load conflict-free across the warp) over the node rows, one
-            // 16-byte broadcast coefficient load per node for 8 FMAs
-            const int ncg = (tk + 63) >> 6, nrb = a.proj_rp >> 2;
-            for (int t = cw; t < ncg * nrb; t += n_cons_warps) {
-                const int cg = t % ncg, rb = t / ncg;
-                const int c = (cg << 6) + lane;
-                if (c >= tk) continue;
-                const unsigned* col = tile + c;
-                const float4* cf = reinterpret_cast<const float4*>(coef) + rb;
-                const int cstep = a.proj_rp >> 2;
-                const bool two = c + 32 < tk;
-                float y0 = 0.f, y1 = 0.f, y2 = 0.f, y3 = 0.f, z0 = 0.f, z1 = 0.f, z2 = 0.f, z3 = 0.f;
-#pragma unroll 4
-                for (int nd = 0; nd < a.n_real; ++nd) {
-                    const float v = Fx<W>::value(col + nd * pitch, hi_off);
-                    const float u = two ? Fx<W>::value(col + nd * pitch + 32, hi_off) : 0.f;
-                    const float4 w = cf[nd * cstep];
-                    y0 = fmaf(w.x, v, y0);
-                    y1 = fmaf(w.y, v, y1);
-                    y2 = fmaf(w.z, v, y2);
-                    y3 = fmaf(w.w, v, y3);
-                    z0 = fmaf(w.x, u, z0);
-                    z1 = fmaf(w.y, u, z1);
-                    z2 = fmaf(w.z, u, z2);
-                    z3 = fmaf(w.w, u, z3);
+        const int rows = tv.l_rows * a.NL;
+        if (a.proj) {
+            const int steps = (rows + 7) >> 3;
+            for (int c = 16 * w; c < tk; c += 16 * fw) {
+                if (a.copies > (W ? 1 : 2)) fold_copies<W, 16>(a, tile, c, rows, lane);
+                for (int nr0 = 0; nr0 < a.proj_nr; nr0 += 3) {   // up to three row blocks in registers
+                    const int nr = a.proj_nr - nr0;
+                    if (!a.proj_frags)
+                        for (int i = 0; i < min(nr, 3); ++i)
+                            project_columns<W, 1, false>(a, steps, first, tile, frag, c, nr0 + i, k_start, tk, inv_fx, lane);
+                    else if (nr >= 3) project_columns<W, 3, true>(a, steps, first, tile, frag, c, nr0, k_start, tk, inv_fx, lane);
+                    else if (nr == 2) project_columns<W, 2, true>(a, steps, first, tile, frag, c, nr0, k_start, tk, inv_fx, lane);
+                    else project_columns<W, 1, true>(a, steps, first, tile, frag, c, nr0, k_start, tk, inv_fx, lane);
                 }
-                const int r = rb << 2;
-                float* dst = a.ldm + (int64_t)r * a.row_stride + k_start + c;
-                const float ys[4] = {y0, y1, y2, y3}, zs[4] = {z0, z1, z2, z3};
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    if (r + i >= a.proj_rows) break;
-                    __stcs(dst + i * a.row_stride, ys[i] * inv_fx);
-                    if (two) __stcs(dst + i * a.row_stride + 32, zs[i] * inv_fx);
-                }
+                zero_columns<W, 16>(a, tile, c, rows, lane);
             }
-            asm volatile("bar.sync 1, %0;" ::"r"(nct) : "memory");   // every read of the tile done
-            zero_tile(tile, n_words, ct, nct);
         } else {
-            // flush the finished tile as floats, word / fx_scale (a power of
-            // two: exact scaling of the rounded word), with plain stores (this
-            // CTA owns its columns), and re-zero it
-            for (int node = cw; node < a.n_nodes; node += n_cons_warps) {
-                unsigned* row = tile + node * pitch;
-                float* dst = a.ldm + node * a.row_stride + k_start;
-                for (int c = lane; c < tk; c += 32) {   // one 128-byte store per warp step
-                    // streaming store: the LDM is read once by the next stage, long after
-                    __stcs(&dst[c], Fx<W>::value(row + c, hi_off) * inv_fx);
-                    row[c] = 0;
-                    if constexpr (W) row[hi_off + c] = 0;
-                }
+            // node rows as floats, word / fx_scale (a power of two: exact
+            // scaling of the rounded word); zero rows outside the tile's
+            const int hi_off = a.rows * a.pitch;
+            for (int c = 32 * w; c < tk; c += 32 * fw) {
+                if (a.copies > 1) fold_copies<W, 32>(a, tile, c, rows, lane);
+                float* dst = a.ldm + k_start + c + lane;
+                const unsigned* src = tile + c + lane;
+                if (c + lane < tk)
+                    for (int n = 0; n < a.n_nodes; ++n) {
+                        const int r = n - first;
+                        const float v = (unsigned)r < (unsigned)rows ? Fx<W>::value(src + r * a.pitch, hi_off) * inv_fx : 0.f;
+                        // streaming store: the LDM is read once by the next stage, long after
+                        __stcs(dst + n * a.row_stride, v);
+                    }
+                zero_columns<W, 32>(a, tile, c, rows, lane);
             }
-            if (a.copies > 1)   // the other copies
-                zero_tile(tile + a.copy_words, n_words - a.copy_words, ct, nct);
         }
-        asm volatile("bar.sync 1, %0;" ::"r"(nct) : "memory");
-    }
-    if (a.in_window) {   // one atomic per warp: per-thread atomics on one word serialise in L2
-        const unsigned tot = __reduce_add_sync(0xffffffffu, counted);
-        if (lane == 0 && tot) atomicAdd(a.in_window, (unsigned long long)tot);
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&tfree[slot]);
     }
 }
 
 template <bool W>
-__global__ void __launch_bounds__(kScatThreads, 1) k_scatter(const ScatterArgs a) {
+__global__ void __launch_bounds__(kScatThreads, 1) k_scatter(const __grid_constant__ ScatterArgs a) {
     scatter_body<W>(a);
 }
 
@@ -706,11 +792,12 @@ __global__ void __launch_bounds__(kScatThreads, 1) k_scatter(const ScatterArgs a
 // shapes of the two variants; the launch covers the larger grid and shared
 // memory (tiles are dealt out by gridDim.x, so the extra CTAs of the smaller
 // variant only take fewer tiles each).
-__global__ void __launch_bounds__(kScatThreads, 1) k_scatter_auto(const ScatterArgs a32, const ScatterArgs a64) {
+__global__ void __launch_bounds__(kScatThreads, 1) k_scatter_auto(const __grid_constant__ ScatterArgs a32,
+                                                                  const __grid_constant__ ScatterArgs a64) {
     if (fx_wide(*a32.cmax))
-        scatter_body<true, 1>(a64);
+        scatter_body<true>(a64);
     else
-        scatter_body<false, 1>(a32);
+        scatter_body<false>(a32);
 }
 
 // ---------------------------------------------------------------------------
@@ -1002,7 +1089,7 @@ __global__ void __launch_bounds__(256) k_gather_grad(const GradArgs g) {
     float acc[3] = {0.f, 0.f, 0.f};
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < g.n_lines; i += stride) {
-        const float2 v = a.v0[i];
+        const float2 v = make_float2(a.vh[i], a.vl[i]);
         const float dl = a.dl ? a.dl[i] : 0.f;
         float fk, tv;
         line_position(a, v, dl, fk, tv);
@@ -1078,7 +1165,7 @@ __global__ void __launch_bounds__(256) k_scatter_tangent(const GradArgs g) {
     const int th = g.theta;
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < g.n_lines; i += stride) {
-        const float2 v = a.v0[i];
+        const float2 v = make_float2(a.vh[i], a.vl[i]);
         const float dl = a.dl ? a.dl[i] : 0.f;
         float fk, tv;
         line_position(a, v, dl, fk, tv);
@@ -1125,17 +1212,18 @@ int check_launch() {
     return e == cudaSuccess ? RG_OK : RG_ERR_CUDA;
 }
 
-int launch_prepare_lines(const double* v0_d, const double* s_d, int64_t n, double c2_tref, float2* v0_out,
-                         float* ls2_out, int* unsorted_flag, cudaStream_t st) {
+int launch_prepare_lines(const double* v0_d, const double* s_d, int64_t n, double c2_tref, float* vh_out,
+                         float* vl_out, float* ls2_out, int* unsorted_flag, cudaStream_t st) {
     if (n <= 0) return RG_OK;
     int64_t blocks = (n + 255) / 256;
-    k_prepare_lines<<<(unsigned)blocks, 256, 0, st>>>(v0_d, s_d, n, c2_tref, v0_out, ls2_out, unsorted_flag);
+    k_prepare_lines<<<(unsigned)blocks, 256, 0, st>>>(v0_d, s_d, n, c2_tref, vh_out, vl_out, ls2_out,
+                                                          unsorted_flag);
     return check_launch();
 }
 
-int launch_col_index(const float2* v0, int64_t n, double vmin, double dv, int c_min, int count,
+int launch_col_index(const float* vh, const float* vl, int64_t n, double vmin, double dv, int c_min, int count,
                      int64_t* col_start, cudaStream_t st) {
-    k_col_index<<<(count + 255) / 256, 256, 0, st>>>(v0, n, vmin, dv, c_min, count, col_start);
+    k_col_index<<<(count + 255) / 256, 256, 0, st>>>(SplitList{vh, vl}, n, vmin, dv, c_min, count, col_start);
     return check_launch();
 }
 

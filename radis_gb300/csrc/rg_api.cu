@@ -1393,7 +1393,17 @@ struct LayoutPlan {
     int m_rows = 0;
 };
 
-int plan_layout(Work& W, const SpecHost& s, cudaStream_t st, LayoutPlan* lp) {
+// The derivatives have no merged rows, so where the spectrum takes those they
+// may take skeleton rows up to 3/4 of the node rows.  Only where the
+// decomposition's frequency samples are fine enough, in front of all: the
+// widest Lorentzian decays by exp(-pi wL f_1) up to the first sample f_1.
+// Largest error of a transform over all frequencies (1e-8 on the samples), 3
+// or 4 x 9 or 16 nodes: 2e-9 .. 6e-7 up to pi wL f_1 = 0.33, 1e-7 .. 3e-5 at
+// 0.65, 1e-3 at 1.3.  10 000 lines, 28 nodes, 12 rows, 400 001 points: three
+// tangents 424 -> 233 us, adjoint's pairs 14 -> 6.
+constexpr double kDerivSkelDecay = 0.25;
+
+int plan_layout(Work& W, const SpecHost& s, cudaStream_t st, LayoutPlan* lp, bool derivs = false) {
     lp->va = std::make_unique<VoigtArgs>();
     lp->vm = std::make_unique<VoigtArgs>();
     lp->vk = std::make_unique<VoigtArgs>();
@@ -1406,9 +1416,15 @@ int plan_layout(Work& W, const SpecHost& s, cudaStream_t st, LayoutPlan* lp) {
     const int alt_rows = merged ? m_rows : s.n_nodes;
     // auto: skeleton rows when no more than the merged rows (whose Gaussian
     // stage costs more than the projection), or 3/4 of the node rows
+    const int limit = lay == 3 ? kProjMaxRows : merged ? alt_rows : 3 * alt_rows / 4;
+    const rg_grid& g = s.grid;
+    const double f1 = 0.5 / W.desc.dv / ((kSkelSamples - 1) * (kSkelSamples - 1));
+    const bool wider = merged && kPi * f1 * std::exp(g.log_wL_min + (g.n_L - 1) * g.dxL) <= kDerivSkelDecay;
+    // (one decomposition for the spectrum and its derivatives)
+    const int limit_d = wider ? std::max(limit, 3 * s.n_nodes / 4) : limit;
     const bool skel = (lay == 0 || lay == 3) &&
-                      plan_skeleton(W, s, *lp->va, lay == 3 ? kProjMaxRows : merged ? alt_rows : 3 * alt_rows / 4,
-                                    lp->vk.get(), &lp->pa, &sk_err);
+                      plan_skeleton(W, s, *lp->va, limit_d, lp->vk.get(), &lp->pa, &sk_err) &&
+                      lp->pa.rows <= (derivs ? limit_d : limit);
     if (skel) merged = false;
     else if (lay == 3) merged = plan_merge(W, s, *lp->va, lp->ga.get(), lp->vm.get(), &m_rows);
     lp->merged = merged;
@@ -1646,7 +1662,7 @@ int enqueue_backward(const rg_lines* L, Work& W, const rg_conditions* c, const S
     // into node rows with the projection coefficients: C restricted to node n
     // is sum_r C[r][n] times skeleton node s_r's convolution)
     LayoutPlan lp;
-    const bool skel = W.desc.layout != 1 && W.desc.layout != 2 && plan_layout(W, s, st, &lp) == RG_OK && lp.skel;
+    const bool skel = W.desc.layout != 1 && W.desc.layout != 2 && plan_layout(W, s, st, &lp, true) == RG_OK && lp.skel;
     if (skel) {
         const VoigtArgs ghat = ar->v;   // keeps g = Ghat
         ar->v = *lp.vk;
@@ -1675,6 +1691,13 @@ int enqueue_backward(const rg_lines* L, Work& W, const rg_conditions* c, const S
     return RG_OK;
 }
 
+// Adds into skeleton rows per float of the node rows and skeleton rows that a
+// projection pass moves, up to which the tangents are scattered straight into
+// the skeleton rows.  28 nodes, 12 rows, 400 001 points, three tangents, with
+// the pass / straight: 10 000 lines 289 / 233 us, 100 000 302 / 247, 400 000 328 /
+// 284, 1 000 000 (1.5 adds per float) 375.5 / 374.
+constexpr double kTangentDirect = 1.25;
+
 // Forward mode: enqueue out + q n_v = d(abscoeff)/d(theta_q) exp(-log_scale_out)
 // for theta = (T, p_bar, x), through the float-LDM tangent scatter and the
 // ordinary FFT / Voigt / inverse FFT stages.
@@ -1686,25 +1709,33 @@ int enqueue_tangent(const rg_lines* L, Work& W, const rg_conditions* c, const Sp
     auto va = std::make_unique<VoigtArgs>();
     fill_voigt_args(W, s, va.get());
     // skeleton layout: each tangent LDM is projected onto the skeleton rows
-    // (in place, tensor cores) before its FFT, as the spectrum's LDM is
+    // (by the scatter, or in place by a pass on the tensor cores) before its FFT
     LayoutPlan lp;
-    const bool skel = W.desc.layout != 1 && W.desc.layout != 2 && plan_layout(W, s, st, &lp) == RG_OK && lp.skel;
+    const bool skel = W.desc.layout != 1 && W.desc.layout != 2 && plan_layout(W, s, st, &lp, true) == RG_OK && lp.skel;
     VoigtArgs& vr = skel ? *lp.vk : *va;
     set_row_shape(W, L->ctx->sms, &vr);
     float* tan = W.ldm;
     ga->tan = tan;
     const int n_v = (int)W.desc.n_v;
+    // straight into the skeleton rows: 2 adds per line and row in the place of 8
+    // and the pass over the node rows
+    const bool direct = skel && 2.0 * lp.pa.rows * (double)L->n <= kTangentDirect * (double)(s.n_nodes + lp.pa.rows) * n_v;
+    if (direct) {
+        ga->proj_coef = lp.pa.coef;
+        ga->proj_rows = lp.pa.rows;
+        ga->proj_rp = lp.pa.rows_pad;
+    }
     for (int q = 0; q < 3; ++q) {
         ga->theta = q;
-        CU(cudaMemsetAsync(tan, 0, sizeof(float) * (size_t)s.n_nodes * W.row_stride, st));
+        CU(cudaMemsetAsync(tan, 0, sizeof(float) * (size_t)(direct ? lp.pa.rows : s.n_nodes) * W.row_stride, st));
         RG(launch_scatter_tangent(*ga, L->ctx->sms * 8, st));
         ColFftArgs ca = col_args(W, s);
-        if (skel) {
+        if (skel) ca.n_pairs = lp.pa.rows / 2;
+        if (skel && !direct) {
             ProjArgs pa = lp.pa;
             pa.ldm = tan;
             pa.sms = L->ctx->sms;
             RG(launch_node_project(pa, st));
-            ca.n_pairs = pa.rows / 2;
         }
         ca.ldm = tan;
         ca.y = W.y;

@@ -384,7 +384,9 @@ struct GradArgs {         // adjoint gather (reverse mode) and tangent scatter (
     double* out;          // gather output: d/dT, d/dp_bar, d/dx sums, zeroed
     // skeleton layout: adj holds the skeleton rows Z_r (r < proj_rows) and a
     // node's adjoint row is sum_r proj_coef[node * proj_rp + r] Z_r (gather);
-    // null: adj holds every node row
+    // null: adj holds every node row.  Tangent: non-null where tan takes the
+    // skeleton rows, row r the sum over nodes of proj_coef[node * proj_rp + r]
+    // x node row
     const float* proj_coef;
     int proj_rows, proj_rp, proj_n;
 };

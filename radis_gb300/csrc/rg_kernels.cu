@@ -1159,7 +1159,8 @@ __global__ void __launch_bounds__(256) k_gather_grad(const GradArgs g) {
 }
 
 // Forward mode: scatter the tangent of each line's 8 LDM values in direction
-// g.theta into the float rows g.tan (FP32 global atomics).
+// g.theta into the float rows g.tan (FP32 global atomics): node rows, or the
+// skeleton rows.
 __global__ void __launch_bounds__(256) k_scatter_tangent(const GradArgs g) {
     const ScatterArgs& a = g.s;
     const int th = g.theta;
@@ -1183,20 +1184,34 @@ __global__ void __launch_bounds__(256) k_scatter_tangent(const GradArgs g) {
         const float Gw[2] = {1.f - tG, tG}, dG[2] = {-r.tG[th], r.tG[th]};
         const float Lw[2] = {1.f - tL, tL}, dL[2] = {-r.tL[th], r.tL[th]};
         const float ln = r.lnI[th];
+        float u[4][2];   // node order (l0, m0), (l0, m0 + 1), (l0 + 1, m0), (l0 + 1, m0 + 1)
 #pragma unroll
-        for (int cl = 0; cl < 2; ++cl)
+        for (int j = 0; j < 4; ++j) {
+            const float gl = Gw[j >> 1] * Lw[j & 1];
+            const float dgl = dG[j >> 1] * Lw[j & 1] + Gw[j >> 1] * dL[j & 1];
 #pragma unroll
-            for (int cm = 0; cm < 2; ++cm) {
-                float* row = g.tan + (int64_t)((l0 + cl) * a.NL + m0 + cm) * g.row_stride + k0;
-                const float gl = Gw[cl] * Lw[cm];
-                const float dgl = dG[cl] * Lw[cm] + Gw[cl] * dL[cm];
+            for (int ck = 0; ck < 2; ++ck) u[j][ck] = I * fmaf(ln, K[ck] * gl, dK[ck] * gl + K[ck] * dgl);
+        }
+        const int n00 = l0 * a.NL + m0;
+        if (g.proj_coef) {
+            const float* c00 = g.proj_coef + n00 * g.proj_rp;
+            const float* c10 = c00 + a.NL * g.proj_rp;
+            float* row = g.tan + k0;
+#pragma unroll 4
+            for (int r = 0; r < g.proj_rows; ++r, row += g.row_stride) {
+                const float c[4] = {__ldg(c00 + r), __ldg(c00 + g.proj_rp + r), __ldg(c10 + r), __ldg(c10 + g.proj_rp + r)};
 #pragma unroll
-                for (int ck = 0; ck < 2; ++ck) {
-                    const float w = K[ck] * gl;
-                    const float dw = dK[ck] * gl + K[ck] * dgl;
-                    atomicAdd(&row[ck], I * fmaf(ln, w, dw));
-                }
+                for (int ck = 0; ck < 2; ++ck)
+                    atomicAdd(&row[ck], fmaf(c[3], u[3][ck], fmaf(c[2], u[2][ck], fmaf(c[1], u[1][ck], c[0] * u[0][ck]))));
             }
+            continue;
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            float* row = g.tan + (int64_t)(n00 + (j >> 1) * a.NL + (j & 1)) * g.row_stride + k0;
+#pragma unroll
+            for (int ck = 0; ck < 2; ++ck) atomicAdd(&row[ck], u[j][ck]);
+        }
     }
 }
 
@@ -1488,13 +1503,13 @@ int launch_gather_grad(const GradArgs& a, int grid, cudaStream_t st) {
     if (a.n_lines <= 0) return RG_OK;
     const size_t smem = a.proj_coef ? sizeof(float) * (size_t)a.proj_n * a.proj_rp : 0;
     ALLOW_SMEM(k_gather_grad, smem);
-    k_gather_grad<<<grid, 256, smem, st>>>(a);
+    k_gather_grad<<<(int)std::min<int64_t>(grid, (a.n_lines + 255) / 256), 256, smem, st>>>(a);
     return check_launch();
 }
 
 int launch_scatter_tangent(const GradArgs& a, int grid, cudaStream_t st) {
     if (a.n_lines <= 0) return RG_OK;
-    k_scatter_tangent<<<grid, 256, 0, st>>>(a);
+    k_scatter_tangent<<<(int)std::min<int64_t>(grid, (a.n_lines + 255) / 256), 256, 0, st>>>(a);
     return check_launch();
 }
 

@@ -417,6 +417,7 @@ __global__ void __launch_bounds__(ColShape<N1>::THREADS, ColShape<N1>::CTAS) k_c
     constexpr int B = ColShape<N1>::B;
     extern __shared__ float4 sm[];
     float4* tws = sm + (N1 > 8 ? N1 * B : 0);
+    chain_begin();
     const int b = threadIdx.x % B;
     const int j = threadIdx.x / B;
     const int c = blockIdx.x * B + b;
@@ -437,8 +438,8 @@ __global__ void __launch_bounds__(ColShape<N1>::THREADS, ColShape<N1>::CTAS) k_c
     for (int q = 0; q < 4; ++q) {
         const int64_t o = (int64_t)(j + q * TPC) * a.n2;
         const bool ok = in && o + 2 * c < a.n_v;
-        v[q].re = ok && na >= 0 ? __ldg(reinterpret_cast<const float2*>(ra + o)) : dup2(0.f);
-        v[q].im = ok && nb >= 0 ? __ldg(reinterpret_cast<const float2*>(rb + o)) : dup2(0.f);
+        v[q].re = ok && na >= 0 ? *reinterpret_cast<const float2*>(ra + o) : dup2(0.f);
+        v[q].im = ok && nb >= 0 ? *reinterpret_cast<const float2*>(rb + o) : dup2(0.f);
     }
 #pragma unroll
     for (int q = 0; q < 4; ++q)   // the sample after an odd n_v's last one is padding
@@ -458,6 +459,7 @@ __global__ void __launch_bounds__(ColShape<N1>::THREADS, ColShape<N1>::CTAS) k_c
     constexpr int B = ColShape<N1>::B;
     extern __shared__ float4 sm[];
     float4* tws = sm + (N1 > 8 ? N1 * B : 0);
+    chain_begin();
     const int b = threadIdx.x % B;
     const int j = threadIdx.x / B;
     const int c = blockIdx.x * B + b;
@@ -482,8 +484,8 @@ __global__ void __launch_bounds__(ColShape<N1>::THREADS, ColShape<N1>::CTAS) k_c
                 off = nidx - (a.n - a.ext);
             }
             if (in && off >= 0) {
-                x[i] = __ldg(&ra[off]);
-                if (rb) z[i] = __ldg(&rb[off]);
+                x[i] = ra[off];
+                if (rb) z[i] = rb[off];
             }
         }
         v[q] = {make_float2(x[0], x[1]), make_float2(z[0], z[1])};
@@ -536,6 +538,7 @@ __global__ void __launch_bounds__(ColShape<N1>::THREADS, ColShape<N1>::CTAS) k_c
     constexpr int B = ColShape<N1>::B;
     extern __shared__ float4 sm[];
     float4* tws = sm + (N1 > 8 ? N1 * B : 0);
+    chain_begin();
     const int b = threadIdx.x % B;
     const int j = threadIdx.x / B;
     const int c = blockIdx.x * B + b;
@@ -573,6 +576,7 @@ __global__ void __launch_bounds__(ColShape<N1>::THREADS, ColShape<N1>::CTAS) k_c
     constexpr int B = ColShape<N1>::B;
     extern __shared__ float4 sm[];
     float4* tws = sm + (N1 > 8 ? N1 * B : 0);
+    chain_begin();
     const int b = threadIdx.x % B;
     const int j = threadIdx.x / B;
     const int c = blockIdx.x * B + b;
@@ -781,6 +785,7 @@ __device__ __forceinline__ void weigh(const A& a, const float4* x, int ub, int j
 template <int CAP>
 __global__ void __launch_bounds__(kRowMaxThreads, 1) k_row_fft_voigt(const RowArgs<CAP> a) {
     extern __shared__ float4 sm4[];
+    chain_begin();
     const FftLen& f = a.f;
     const int h = f.L;
     const int ub = f.row_len;
@@ -830,6 +835,7 @@ __device__ __forceinline__ void weigh_adj(const A& a, float4* out, int ub, int j
 template <int CAP>
 __global__ void __launch_bounds__(kRowMaxThreads, 1) k_row_ifft_adj(const RowArgs<CAP> a) {
     extern __shared__ float4 sm4[];
+    chain_begin();
     const FftLen& f = a.f;
     const int h = f.L;
     const int ub = f.row_len;
@@ -851,8 +857,7 @@ __global__ void __launch_bounds__(kRowMaxThreads, 1) k_row_ifft_adj(const RowArg
 template <int N1, class K>
 static int launch_col(K kernel, const ColFftArgs& a, int pairs, cudaStream_t st) {
     dim3 grid((a.n2 / 2 + ColShape<N1>::B - 1) / ColShape<N1>::B, pairs);
-    kernel<<<grid, ColShape<N1>::THREADS, ColShape<N1>::SMEM, st>>>(a);
-    return check_launch();
+    return launch_chained(kernel, grid, ColShape<N1>::THREADS, ColShape<N1>::SMEM, st, a);
 }
 #define RG_COL(name, fn, pairs)                                             \
     template <int N1>                                                       \
@@ -931,12 +936,10 @@ static int launch_row(const VoigtArgs& v, float4* adj_out, cudaStream_t st) {
     const size_t smem = row_smem(v.f2, v.units, !adj && v.units < v.n_pairs);
     if (adj) {
         ALLOW_SMEM(k_row_ifft_adj<CAP>, smem);
-        k_row_ifft_adj<CAP><<<dim3(v.n1, (v.n_pairs + v.units - 1) / v.units), v.threads, smem, st>>>(a);
-    } else {
-        ALLOW_SMEM(k_row_fft_voigt<CAP>, smem);
-        k_row_fft_voigt<CAP><<<v.n1, v.threads, smem, st>>>(a);
+        return launch_chained(k_row_ifft_adj<CAP>, dim3(v.n1, (v.n_pairs + v.units - 1) / v.units), v.threads, smem, st, a);
     }
-    return check_launch();
+    ALLOW_SMEM(k_row_fft_voigt<CAP>, smem);
+    return launch_chained(k_row_fft_voigt<CAP>, v.n1, v.threads, smem, st, a);
 }
 static int launch_row_any(const VoigtArgs& v, float4* adj_out, cudaStream_t st) {
     if (v.f2.L != v.n2 / 2 || v.f2.npass < 2 || v.units < 1 || v.threads < 32 || v.threads > kRowMaxThreads || v.threads % 32 ||

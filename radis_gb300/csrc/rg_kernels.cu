@@ -610,18 +610,6 @@ __device__ __forceinline__ void scatter_body(const ScatterArgs& a) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int lw = a.line_warps, fw = (int)(blockDim.x >> 5) - 1 - lw;
 
-    if (nq > a.rng_cap) {   // the host sizes the table for every CTA: never taken
-        if (threadIdx.x == 0) atomicExch(a.err, 1u);
-        return;
-    }
-    auto col_idx = [&](int c) { return max(0, min(c + a.col_off, a.col_count - 1)); };
-    for (int q = threadIdx.x; q < nq; q += blockDim.x) {
-        const int k_start = ((int)blockIdx.x + q * G) * a.TK;
-        const int tk = min(a.TK, a.n_v - k_start);
-        const int lo = (int)a.col_start[col_idx(k_start - 1 - a.margin_cols)];
-        const int hi = (int)a.col_start[col_idx(k_start + tk + a.margin_cols)];
-        rng[q] = make_int2(lo / kLinePad * kLinePad, hi);   // 16-line aligned start
-    }
     {
         uint4* z = reinterpret_cast<uint4*>(tiles - 4);   // with the words before the first tile
         for (int i = threadIdx.x; i <= a.slots * slot_words / 4; i += blockDim.x) z[i] = make_uint4(0u, 0u, 0u, 0u);
@@ -637,6 +625,19 @@ __device__ __forceinline__ void scatter_body(const ScatterArgs& a) {
         }
         mbar_init(fmeet, fw);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    chain_begin();
+    if (nq > a.rng_cap) {   // the host sizes the table for every CTA: never taken
+        if (threadIdx.x == 0) atomicExch(a.err, 1u);
+        return;
+    }
+    auto col_idx = [&](int c) { return max(0, min(c + a.col_off, a.col_count - 1)); };
+    for (int q = threadIdx.x; q < nq; q += blockDim.x) {
+        const int k_start = ((int)blockIdx.x + q * G) * a.TK;
+        const int tk = min(a.TK, a.n_v - k_start);
+        const int lo = (int)a.col_start[col_idx(k_start - 1 - a.margin_cols)];
+        const int hi = (int)a.col_start[col_idx(k_start + tk + a.margin_cols)];
+        rng[q] = make_int2(lo / kLinePad * kLinePad, hi);   // 16-line aligned start
     }
     __syncthreads();
 
@@ -794,6 +795,7 @@ __global__ void __launch_bounds__(kScatThreads, 1) k_scatter(const __grid_consta
 // variant only take fewer tiles each).
 __global__ void __launch_bounds__(kScatThreads, 1) k_scatter_auto(const __grid_constant__ ScatterArgs a32,
                                                                   const __grid_constant__ ScatterArgs a64) {
+    chain_begin();
     if (fx_wide(*a32.cmax))
         scatter_body<true>(a64);
     else
@@ -915,6 +917,7 @@ __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_gr
 
 __global__ void __launch_bounds__(256) k_gauss_merge(const GaussArgs a) {
     extern __shared__ __align__(16) float gsm[];
+    chain_begin();
     constexpr int TW = kGaussTile;
     constexpr int P = kGaussPer;                     // outputs per thread (8)
     constexpr int S = kGaussStages;
@@ -1253,19 +1256,16 @@ int launch_col_cmax(const int64_t* col_start, int col_off, int col_count, int n_
 int launch_scatter(const ScatterArgs& a, int grid, int threads, size_t smem, bool wide, cudaStream_t st) {
     if (wide) {
         ALLOW_SMEM(k_scatter<true>, smem);
-        k_scatter<true><<<grid, threads, smem, st>>>(a);
-    } else {
-        ALLOW_SMEM(k_scatter<false>, smem);
-        k_scatter<false><<<grid, threads, smem, st>>>(a);
+        return launch_chained(k_scatter<true>, grid, threads, smem, st, a);
     }
-    return check_launch();
+    ALLOW_SMEM(k_scatter<false>, smem);
+    return launch_chained(k_scatter<false>, grid, threads, smem, st, a);
 }
 
 int launch_scatter_auto(const ScatterArgs& a32, const ScatterArgs& a64, int grid, int threads, size_t smem,
                         cudaStream_t st) {
     ALLOW_SMEM(k_scatter_auto, smem);
-    k_scatter_auto<<<grid, threads, smem, st>>>(a32, a64);
-    return check_launch();
+    return launch_chained(k_scatter_auto, grid, threads, smem, st, a32, a64);
 }
 
 // Dynamic shared memory a scatter variant may have (one CTA per SM).
@@ -1473,8 +1473,7 @@ int launch_gauss_merge(const GaussArgs& a0, int out_rows, cudaStream_t st) {
     const size_t smem = sizeof(float) * (size_t)kGaussStages * a.slot_len;
     ALLOW_SMEM(k_gauss_merge, smem);
     dim3 grid((Lr + kGaussTile - 1) / kGaussTile, out_rows);
-    k_gauss_merge<<<grid, 256, smem, st>>>(a);
-    return check_launch();
+    return launch_chained(k_gauss_merge, grid, 256, smem, st, a);
 }
 
 // Threads per group of the slit convolution: the outputs dealt out in the

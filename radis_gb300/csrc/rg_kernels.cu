@@ -538,10 +538,20 @@ __device__ __forceinline__ void project_columns(const ScatterArgs& a, int steps,
         for (int i = 0; i < 4; ++i) d[nr][i] = e[nr][i] = 0.f;
 #pragma unroll 2
     for (int s = 0; s < steps; ++s, col += 8 * a.pitch, cf += 32 * a.proj_nr) {
+        const unsigned* p[4] = {col, col + 8, col + a.pitch, col + a.pitch + 8};
+        {   // Leave out nodes and columns that hold nothing: 0 x coefficient.  A
+            // line fills 4 of a window's nodes, so in a 5M-line list of 12 lines
+            // per column and in sparser ones many steps are empty (spectrum 114 ->
+            // 108 us; 0.03 lines per column 41.2 -> 38.8, 100M lines 1214 -> 1164 us).
+            // Loading the next step's words before this one's MMAs as well: 117 us.
+            unsigned any = p[0][0] | p[1][0] | p[2][0] | p[3][0];
+            if (W) any |= p[0][hi_off] | p[1][hi_off] | p[2][hi_off] | p[3][hi_off];
+            if (two) any |= p[0][a.copy_words] | p[1][a.copy_words] | p[2][a.copy_words] | p[3][a.copy_words];
+            if (!__any_sync(0xffffffffu, any)) continue;
+        }
         float4 b[NR];
 #pragma unroll
         for (int nr = 0; nr < NR; ++nr) b[nr] = kFrags ? cf[nr * 32] : proj_frag(a, nr0 + nr, first + 8 * s, lane);
-        const unsigned* p[4] = {col, col + 8, col + a.pitch, col + a.pitch + 8};
         uint32_t ah[4], al[4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
@@ -589,10 +599,11 @@ __device__ __forceinline__ void project_columns(const ScatterArgs& a, int steps,
 // grid's: 12 x 24 nodes need 72 of 288 rows, so that two tiles of hundreds of
 // columns fit and the flush reads a quarter.  One kernel projects every grid:
 // the node rows never reach memory.  Against one tile of all rows filled and
-// flushed in turn: 5M lines x 400k points 94 -> 57 us (28 bytes a line are 21
+// flushed in turn: 5M lines x 400k points 94 -> 55 us (28 bytes a line are 21
 // us of HBM; the shared atomics' wavefronts, the flush's MMA chains and its
 // last tile are the rest), 100M x 1.5M points 1130 + 407 (a projection pass) ->
-// 800 us (HBM: 414 us).  Two CTAs per SM of half the size: 58.6 and 957 us.
+// 760 us (HBM: 414 us).  Two CTAs per SM of half the size: 58.6 and 957 us where
+// one took 57 and 800.
 template <bool W>
 __device__ __forceinline__ void scatter_body(const ScatterArgs& a) {
     extern __shared__ __align__(128) unsigned char smem[];

@@ -71,3 +71,24 @@ def test_scatter_windows(ctx, masses, n_v, dv, vmin, per_col, n_G, n_L, accumula
     ln.close()
     assert ia.accum_bits == ib.accum_bits == accumulator and np.array_equal(b, c)
     assert np.max(np.abs(a - b)) <= 2e-5 * np.max(np.abs(a)), (ib.layout, ib.fft_rows)
+
+
+@pytest.mark.parametrize("accumulator", [32, 64])
+@pytest.mark.parametrize("columns", [[0], [15], [16, 17], [5, 700, 9_998], [9_999]])
+def test_mostly_empty_columns(ctx, columns, accumulator):
+    """A few lines in a window of empty columns: the projection leaves out the
+    columns and nodes that hold nothing.  Skeleton against node rows, 2e-5 of
+    the peak; nothing at all where the only line lies on the last column."""
+    vmin, dv, n_v = 2000.0, 0.01, 10_000
+    lines = S.uniform_lines(200, vmin + 200.0, vmin + 400.0, seed=3, s_lo=1e-21, s_hi=1e-20, el_mean=1.0)
+    lines["v0"][:len(columns)] = vmin + dv * (np.array(columns) + 0.3)   # the others span the node axes
+    ln = L.Lines(ctx, lines, 44.0)
+    out = []
+    for layout in (1, 3):
+        plan = L.Plan(ln, vmin, dv, n_v, n_G=6, n_L=9, accumulator=accumulator, layout=layout)
+        out.append(plan.synthesize_host(900.0, 0.5, 0.2))
+        plan.close()
+    ln.close()
+    (a, _), (b, i) = out
+    assert i.layout == 4 and (np.max(a) > 0) == (columns[0] + 1 < n_v)
+    assert np.max(np.abs(a - b)) <= 2e-5 * np.max(np.abs(a))

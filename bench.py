@@ -49,28 +49,35 @@ WORKLOAD = "co2_5M"
 KERNELS_PER_STEP = 5   # plain layout: scatter, column FFT, row FFT + Voigt, inverse row, inverse column
 
 
-def inverse_fused(info):
-    """The inverse row DFT runs inside the forward row kernel when one CTA
-    holds a row's whole pair sum (at most 16 pairs, i.e. 32 FFT rows)."""
-    return int(info.fft_rows) // 2 <= 16
-
-
 def kernels_per_step(info):
-    """Kernels one spectrum launches: scatter, column FFT, row FFT + Voigt,
-    inverse row FFT (unless fused into the row kernel) and inverse column
-    FFT; with the skeleton layout the projection in addition (none when the
-    scatter projects); with the merged layout the Gaussian stage and the
-    merged-row column FFT instead of the column FFT, plus a column FFT of the
-    narrow-node rows when there are any."""
-    base = KERNELS_PER_STEP - (1 if inverse_fused(info) else 0)
+    """Steps of one spectrum's stage list: scatter, column FFT, row FFT +
+    Voigt, inverse row FFT (counted up to 16 pairs of rows with the row FFT)
+    and inverse column FFT; skeleton rows of a grid of more than 160 nodes
+    count their projection, merged rows the Gaussian stage and the column FFT
+    of the narrow-node rows when there are any."""
+    base = KERNELS_PER_STEP - (1 if int(info.fft_rows) // 2 <= 16 else 0)
     if int(info.layout) == 3:
         return base + 1
     if int(info.layout) == 4 or not info.merged_rows:
         return base
     nlv = info.merged_rows + (info.merged_rows & 1)
     return base + 1 + (1 if info.fft_rows > nlv else 0)
-STAGES = ["k_scatter", "k_col_fft_fwd", "k_row_fft_voigt", "k_row_ifft", "k_col_ifft"]
-LAYOUT_NAMES = {1: "node rows", 2: "merged rows", 3: "skeleton rows", 4: "skeleton rows, projected in the scatter"}
+
+
+def launches_per_step(info):
+    """Kernels one spectrum launches: scatter (which projects onto the
+    skeleton rows), column FFT, row FFT + Voigt + inverse row FFT and inverse
+    column FFT; with merged rows the Gaussian stage and, where there are
+    narrow-node rows, a column FFT of theirs in addition."""
+    if int(info.layout) in (3, 4) or not info.merged_rows:
+        return 4
+    nlv = info.merged_rows + (info.merged_rows & 1)
+    return 5 + (1 if info.fft_rows > nlv else 0)
+
+
+STAGES = ["k_scatter", "k_col_fft_fwd", "k_row_fft_voigt", None, "k_col_ifft"]   # by stage event; 3 is part of 2
+LAYOUT_NAMES = {1: "node rows", 2: "merged rows", 3: "skeleton rows, projected in the scatter (more than 160 nodes)",
+                4: "skeleton rows, projected in the scatter"}
 
 
 # name: (label, lines factory, molar mass, vmin, vmax, wstep, T, p_bar, x, n_G, n_L)
@@ -183,23 +190,19 @@ def algorithmic_bytes(n_lines_read, line_bytes, n_nodes, n_v, n_ft, info):
     """Bytes each kernel must move once (per spectrum): the line records
     (``line_bytes`` each) and the LDM written once (n_v columns, no zero
     padding); the column FFT reads its node rows and writes the packed complex
-    rows; the row stage reads them (its accumulator G is stored once); the
-    inverse stages read/write G and the output.  With the merged layout the
+    rows; the row stage reads them and stores G once, after its inverse part;
+    the inverse column stage reads G and writes the output.  With the merged layout the
     Gaussian stage reads the wide-node LDM rows and writes the n_L merged rows
     (n_v + 2 ext points), and the column FFT reads those and the narrow-node
-    rows.  With the skeleton layout the projection reads the node rows and
-    writes the skeleton rows, which the column FFT reads; projected in the
-    scatter's flush, the scatter writes only the skeleton rows."""
+    rows.  With the skeleton layout the scatter writes only the skeleton
+    rows, which the column FFT reads."""
     pairs = int(info.fft_rows or n_nodes) // 2
     out = {
         "k_scatter": n_lines_read * line_bytes + n_nodes * n_v * 4,
         "k_col_fft_fwd": n_nodes * n_v * 4 + pairs * n_ft * 8,
         "k_row_fft_voigt": pairs * n_ft * 8 + n_ft * 8,
-        "k_row_ifft": 2 * n_ft * 8,
         "k_col_ifft": n_ft * 8 + n_v * 4,
     }
-    if inverse_fused(info):   # G written once, after the inverse part
-        out.pop("k_row_ifft")
     NL = int(info.merged_rows)
     if NL:
         nlv = NL + (NL & 1)
@@ -210,12 +213,8 @@ def algorithmic_bytes(n_lines_read, line_bytes, n_nodes, n_v, n_ft, info):
         out["k_col_fft_fwd"] = merged + n_narrow * NL * n_v * 4 + pairs * n_ft * 8
     if int(info.layout) in (3, 4):
         rows = int(info.fft_rows)
-        real_nodes = int(info.grid.n_G) * int(info.grid.n_L)
         out["k_col_fft_fwd"] = rows * n_v * 4 + pairs * n_ft * 8
-        if int(info.layout) == 3:
-            out["k_node_project"] = real_nodes * n_v * 4 + rows * n_v * 4
-        else:   # projected by the scatter's flush: only the skeleton rows are written
-            out["k_scatter"] = n_lines_read * line_bytes + rows * n_v * 4
+        out["k_scatter"] = n_lines_read * line_bytes + rows * n_v * 4
     return out
 
 
@@ -695,15 +694,10 @@ def time_plan(plan, T, p, x, n_v, K, stream, warm=3):
 
 def kernel_times(stage_avg, gauss, info):
     """Per-kernel ms from the stage events: with the merged layout the column
-    stage is the Gaussian stage (its own event) followed by the column FFT,
-    with the skeleton layout the projection followed by the column FFT."""
-    kt = {STAGES[i]: stage_avg[i] for i in range(5)}
-    if inverse_fused(info):   # one kernel: its stage ends after its inverse part
-        kt["k_row_fft_voigt"] += kt.pop("k_row_ifft")
-    if int(info.layout) == 3:
-        kt["k_node_project"] = gauss
-        kt["k_col_fft_fwd"] = stage_avg[1] - gauss
-    elif info.merged_rows:
+    stage is the Gaussian stage (its own event) followed by the column FFT."""
+    kt = {STAGES[i]: stage_avg[i] for i in range(5) if STAGES[i]}
+    kt["k_row_fft_voigt"] += stage_avg[3]   # one kernel: its stage ends after its inverse part
+    if info.merged_rows:
         kt["k_gauss_merge"] = gauss
         kt["k_col_fft_fwd"] = stage_avg[1] - gauss
     return kt
@@ -873,7 +867,7 @@ def run_ours(args):
             "vs_baseline": None, "dtype": "f32", "data": "synthetic",
             "config": workload_desc(wl, n_lines, n_v, lb),
             "clocks": clk.summary(),
-            "gpu_launches": kernels_per_step(info) * K,
+            "gpu_launches": launches_per_step(info) * K,
             "e2e": {"value": ws * 1000.0 / e2e_ms, "unit": "spectra/s",
                     "h2d_bytes_per_step": 0, "d2h_bytes_per_step": n_v * 4,
                     "note": ("resident line list (as the reference's gpuApp.iterate); per step the conditions "
@@ -900,13 +894,13 @@ def run_ours(args):
                            "skeleton_sampled_err": float(info.layout_err)},
             "setup_s": setup_s,
         }
-        if name == "k_scatter" and int(info.layout) == 4:
+        if name == "k_scatter" and int(info.layout) in (3, 4):
             res["roofline"]["note"] = (
                 "the scatter writes only the skeleton rows: each finished tile is projected onto them in shared "
-                f"memory ({g.n_G * g.n_L} x {int(info.fft_rows)} FMA per grid column), so the kernel moves "
+                f"memory, so the kernel moves "
                 f"{ab[name] / 1e6:.0f} MB instead of {(lines_in_window * lb + n_nodes * n_v * 4) / 1e6:.0f} MB "
-                "and is bound by its instruction issue, not HBM; frac is the HBM fraction of the bytes it must "
-                "move")
+                "and is bound by its shared-memory atomics and the projection, not HBM; frac is the HBM fraction of "
+                "the bytes it must move")
         if name == "k_gauss_merge":
             res["roofline"]["note"] = ("the real-space Gaussian stage is FP32-FMA-bound (a banded convolution of "
                                        "each wide-node row with its residual Gaussian, ~200 FMA per merged "
@@ -937,8 +931,7 @@ def run_ours(args):
         if ws == 1 and not args.no_fft_compare:
             fwd = kt["k_col_fft_fwd"] + kt["k_row_fft_voigt"]
             res["fft_vs_cufft"] = {wl: run_fft_compare(int(g.n_ft), int(info.fft_rows or n_nodes), fwd,
-                                                       kt.get("k_row_ifft", 0.0) + kt["k_col_ifft"],
-                                                       inverse_row_in_forward="k_row_ifft" not in kt)}
+                                                       kt["k_col_ifft"], inverse_row_in_forward=True)}
         if ws == 1 and not args.no_slit:
             plan.synthesize_device(T, p, x, out.data_ptr(), torch.cuda.current_stream().cuda_stream or 1)
             res["slit"] = run_slit(ctx, out, vmin, dv)
@@ -955,8 +948,7 @@ def run_ours(args):
                 c3_rows = c3["fft_layout"]["fft_rows"]
                 res.setdefault("fft_vs_cufft", {})["h2o_100M"] = run_fft_compare(
                     c3["fft_layout"]["n_ft"], c3_rows, kt3["k_col_fft_fwd"] + kt3["k_row_fft_voigt"],
-                    kt3.get("k_row_ifft", 0.0) + kt3["k_col_ifft"], reps=5,
-                    inverse_row_in_forward="k_row_ifft" not in kt3)
+                    kt3["k_col_ifft"], reps=5, inverse_row_in_forward=True)
             res["c3"] = c3
         if h2o_host is not None:
             h2o_host = None

@@ -169,10 +169,10 @@ struct Work {
     float* mrow = nullptr;
     size_t mrow_bytes = 0;
     int last_fft_rows = 0, last_merged_rows = 0, last_ext = 0;   // layout of the last spectrum
-    int last_layout = 0;              // 1 node rows, 2 merged rows, 3 skeleton rows
+    int last_layout = 0;              // 1 node rows, 2 merged rows, 3 skeleton rows, 4 those of at most 160 nodes
     double last_layout_err = 0.0;     // skeleton layout: the decomposition's sampled error
-    // skeleton layout: projection coefficients [n_nodes][rows_pad] (device,
-    // grow-only) and their host staging (copied from pageable memory: the
+    // skeleton layout: projection coefficients and fragments (plan_skeleton;
+    // device, grow-only) and their host staging (copied from pageable memory: the
     // copy has left this buffer when cudaMemcpyAsync returns)
     bool allow_skeleton = true;
     bool proj_fixed = false;          // proj_coef is a fixed piece of scratch (never reallocated)
@@ -1098,7 +1098,6 @@ bool plan_merge(const Work& W, const SpecHost& s, const VoigtArgs& va, GaussArgs
     ga->out_stride = (ga->n_v + 2 * K_max + 31) / 32 * 32;
     ga->ldm = W.ldm;
     ga->row_stride = W.row_stride;
-    ga->cmax = W.cmax_dev;
     *vm = va;
     vm->n_nodes = *out_rows;
     vm->n_pairs = *out_rows / 2;
@@ -1504,7 +1503,6 @@ int enqueue_spectrum(const rg_lines* L, Work& W, const rg_conditions* c, const S
         ca.row_stride = W.row_stride;
         ca.n_pairs = s.n_nodes / 2;
         ca.ldm = W.ldm;
-        ca.cmax = W.cmax_dev;
         ca.y = W.y;
         ca.tw_hi = W.tw_hi;
         ca.tw_lo = W.tw_lo;

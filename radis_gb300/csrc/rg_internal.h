@@ -221,7 +221,6 @@ struct ColFftArgs {       // K2 (forward column FFT) and K4 (inverse column FFT)
     int64_t row_stride;
     int n_pairs;
     const float* ldm;     // K2 input: the scatter's LDM [node][row_stride]
-    const int* cmax;      // device: fixed-point bound of the scatter (scale = fx_scale(*cmax))
     float4* y;            // K2 output [pair][n1][n2 / 2], columns 2c, 2c + 1 per element
     const float2* tw_hi;  // exp(-2 pi i 1024 t / N)
     const float2* tw_lo;  // exp(-2 pi i t / N), t < 1024
@@ -279,10 +278,12 @@ struct VoigtArgs {        // K3 (row FFT + Voigt weights + pair reduction + inve
 // their Gaussian kernel and summed into one row per wL node (the other,
 // narrow-Gaussian node rows stay in the LDM).  Output rows [m][out_stride]
 // hold k in [-ext, n_v + ext) at offset k + ext.
-// Skeleton layout: the LDM rows projected, in place, onto the rows of a few
-// skeleton nodes whose transforms span every node's (interp_decomp):
+// Skeleton layout: the LDM rows projected onto the rows of a few skeleton nodes
+// whose transforms span every node's (interp_decomp):
 // row r (r < rows) <- sum_n coef[n * rows_pad + r] x row n, column by column;
-// rows [R, rows) of an odd R are the zero pad row.
+// rows [R, rows) of an odd R are the zero pad row.  The scatter projects as it
+// flushes (flush); the tangents of dense lists have a pass of their own, in
+// place (frag).
 constexpr int kProjMaxRows = 64;
 struct ProjArgs {
     float* ldm;           // LDM [node][row_stride], rows [0, rows) overwritten
@@ -293,10 +294,10 @@ struct ProjArgs {
     int rows_pad;         // coefficient row pitch (the kernel's row block)
     const float* coef;    // [n_nodes][rows_pad]
     int sms;              // SMs of the device (persistent grid)
-    // tensor-core form: the coefficients as TF32 hi / lo parts in the B
+    // the pass: the coefficients as TF32 hi / lo parts in the B
     // fragments of mma.m16n8k8 (rows in blocks of 8, nodes in steps of 8):
     // frag[((nr * ksteps + ks) * 2 + part) * 64 + lane * 2 + i]
-    const float* frag;    // null: FP32 pass
+    const float* frag;
     int mtiles;           // row blocks of 8 (<= 8)
     int ksteps;           // node steps of 8 in frag (a multiple of 2)
     // the scatter's flush (ScatterArgs::proj): the coefficients' (hi, lo) parts,
@@ -322,7 +323,6 @@ constexpr int kGaussMaxK = 256;       // widest kernel half-width (points)
 struct GaussArgs {
     const float* ldm;     // LDM [node][row_stride]
     int64_t row_stride;
-    const int* cmax;      // fixed-point bound (scale)
     float* out;
     int64_t out_stride;
     int n_v, ext, NL;

@@ -734,10 +734,11 @@ int scatter_shape(const rg_lines* L, const Work& W, const SpecHost& s, bool wide
     const double lines_per_col = mean_lines_per_col(L, W.desc.dv);
     // the working warps shared out by the instructions per column of the two
     // jobs: ~80 per 32 lines; a flush step of 8 nodes x 16 columns ~45 and its
-    // MMAs, or a store per node row.  Scatter over 7 / 9 / 11 / 13 / 15 / 17 /
-    // 19 line warps: 14.6 lines per column (5M) 70 / 64 / 60 / 59 / 58 / 68 / 75
-    // us, 67 (100M) 1063 / 968 / 834 / 858 / 816 / 799 / 856, 0.03 (10 000)
-    // 17.2 / 16.5 / 17.4 / 18.2 / 20 / 22 / 26
+    // MMAs, or a store per node row.  Scatter over 11 / 13 / 15 / 17 / 19 line
+    // warps (chosen in brackets): 12.5 lines per column (5M) 57.4 / [55.6] / 55.7 /
+    // 64 / - us, 67 (100M) - / - / 770 / [759] / 802; over 7 / 9 / 11 / 13 / 15 of
+    // them, the flush as it was before it left out empty steps: 0.05 (10 000)
+    // 17.2 / [16.5] / 17.4 / 18.2 / 20, now 15.0.
     const int win256 = tile_rows_needed(L, W, s, 256);
     const double flush = fuse ? ((win256 * NL + 7) / 8 * (40.0 + 6.0 * fuse->flush_nr) + 80.0) / 16.0 : 0.25 * s.n_nodes;
     const double line = 2.5 * lines_per_col + 2.0;
